@@ -689,6 +689,55 @@ __device__ __forceinline__ void from_face(const R f[6], int d, R out[5]) {
   else { out[3] = f[1]; out[1] = f[3]; out[2] = f[4]; }
 }
 
+// The 8 children of one variable: a[0] the father cell's value, a[1..6] its
+// neighbours' (-x,+x,-y,+y,-z,+z), t the interpol_type of that variable.
+__device__ __forceinline__ void interp_one_var(const double a[7], int t, double out[8]) {
+  double w[3] = {0.0, 0.0, 0.0};
+  if (t == 1) {  // compute_limiter_minmod :449-476
+    for (int idim = 1; idim <= 3; idim++) {
+      double dl = 0.5 * (a[2 * idim] - a[0]);
+      double dr = 0.5 * (a[0] - a[2 * idim - 1]);
+      double mm;
+      if (dl * dr <= 0.0) mm = 0;
+      else mm = fmn(fabs(dl), fabs(dr)) * dl / fabs(dl);
+      w[idim - 1] = mm;
+    }
+  } else if (t == 3) {  // compute_central :618-637
+    for (int idim = 1; idim <= 3; idim++) w[idim - 1] = 0.25 * (a[2 * idim] - a[2 * idim - 1]);
+  } else if (t == 2) {  // compute_limiter_central :481-613
+    for (int idim = 1; idim <= 3; idim++) w[idim - 1] = 0.25 * (a[2 * idim] - a[2 * idim - 1]);
+    double ac[8];
+    for (int ind = 0; ind < 8; ind++) ac[ind] = a[0];
+    for (int idim = 0; idim < 3; idim++)
+      for (int ind = 0; ind < 8; ind++) {
+        double xc = (double)((ind >> idim) & 1) - 0.5;
+        ac[ind] = ac[ind] + 2.0 * w[idim] * xc;
+      }
+    double corner = ac[0];
+    for (int j = 1; j < 8; j++) corner = fmx(corner, ac[j]);
+    double kernel = a[1];
+    for (int j = 2; j <= 6; j++) kernel = fmx(kernel, a[j]);
+    double dk = a[0] - kernel, dc = a[0] - corner;
+    double max_lim = 0.0;
+    if (dk * dc > 0.0) max_lim = fmn(1.0, dk / dc);
+    corner = ac[0];
+    for (int j = 1; j < 8; j++) corner = fmn(corner, ac[j]);
+    kernel = a[1];
+    for (int j = 2; j <= 6; j++) kernel = fmn(kernel, a[j]);
+    dk = a[0] - kernel;
+    dc = a[0] - corner;
+    double min_lim = 0.0;
+    if (dk * dc > 0.0) min_lim = fmn(1.0, dk / dc);
+    double lim = fmn(min_lim, max_lim);
+    for (int idim = 0; idim < 3; idim++) w[idim] = w[idim] * lim;
+  }
+  for (int ind = 0; ind < 8; ind++) {
+    double v = a[0];
+    for (int idim = 0; idim < 3; idim++) v = v + w[idim] * ((double)((ind >> idim) & 1) - 0.5);
+    out[ind] = v;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Coarse-to-fine prolongation of one child (interpol_hydro,
 // interpol_hydro.f90:268-637). u7[j][v]: father cell (j=0) and its 6
@@ -711,53 +760,10 @@ __device__ __forceinline__ void interp_children(double u1[7][5], const rb_hydro_
     }
   }
   for (int iv = 0; iv < 5; iv++) {
-    double a[7], w[3] = {0.0, 0.0, 0.0};
+    double a[7], o[8];
     for (int j = 0; j <= 6; j++) a[j] = u1[j][iv];
-    int t = itype;
-    if (itype == 4) t = (iv >= 1 && iv <= 3) ? 3 : 2;
-    if (t == 1) {  // compute_limiter_minmod :449-476
-      for (int idim = 1; idim <= 3; idim++) {
-        double dl = 0.5 * (a[2 * idim] - a[0]);
-        double dr = 0.5 * (a[0] - a[2 * idim - 1]);
-        double mm;
-        if (dl * dr <= 0.0) mm = 0;
-        else mm = fmn(fabs(dl), fabs(dr)) * dl / fabs(dl);
-        w[idim - 1] = mm;
-      }
-    } else if (t == 3) {  // compute_central :618-637
-      for (int idim = 1; idim <= 3; idim++) w[idim - 1] = 0.25 * (a[2 * idim] - a[2 * idim - 1]);
-    } else if (t == 2) {  // compute_limiter_central :481-613
-      for (int idim = 1; idim <= 3; idim++) w[idim - 1] = 0.25 * (a[2 * idim] - a[2 * idim - 1]);
-      double ac[8];
-      for (int ind = 0; ind < 8; ind++) ac[ind] = a[0];
-      for (int idim = 0; idim < 3; idim++)
-        for (int ind = 0; ind < 8; ind++) {
-          double xc = (double)((ind >> idim) & 1) - 0.5;
-          ac[ind] = ac[ind] + 2.0 * w[idim] * xc;
-        }
-      double corner = ac[0];
-      for (int j = 1; j < 8; j++) corner = fmx(corner, ac[j]);
-      double kernel = a[1];
-      for (int j = 2; j <= 6; j++) kernel = fmx(kernel, a[j]);
-      double dk = a[0] - kernel, dc = a[0] - corner;
-      double max_lim = 0.0;
-      if (dk * dc > 0.0) max_lim = fmn(1.0, dk / dc);
-      corner = ac[0];
-      for (int j = 1; j < 8; j++) corner = fmn(corner, ac[j]);
-      kernel = a[1];
-      for (int j = 2; j <= 6; j++) kernel = fmn(kernel, a[j]);
-      dk = a[0] - kernel;
-      dc = a[0] - corner;
-      double min_lim = 0.0;
-      if (dk * dc > 0.0) min_lim = fmn(1.0, dk / dc);
-      double lim = fmn(min_lim, max_lim);
-      for (int idim = 0; idim < 3; idim++) w[idim] = w[idim] * lim;
-    }
-    for (int ind = 0; ind < 8; ind++) {
-      double v = a[0];
-      for (int idim = 0; idim < 3; idim++) v = v + w[idim] * ((double)((ind >> idim) & 1) - 0.5);
-      u2[ind][iv] = v;
-    }
+    interp_one_var(a, itype == 4 ? ((iv >= 1 && iv <= 3) ? 3 : 2) : itype, o);
+    for (int ind = 0; ind < 8; ind++) u2[ind][iv] = o[ind];
   }
   if (ivar_ == 1 || ivar_ == 2) {
     if (ivar_ == 2) {

@@ -256,6 +256,31 @@ static __global__ void interp_blocks_kernel(const double* __restrict__ uold, con
     for (int v = 0; v < 5; v++) out[v * stride + (int64_t)e * 8 + ind] = u2[ind][v];
 }
 
+// The same for interpol_var = 0, where no variable depends on another: one
+// thread per (entry, variable), blockIdx.y the variable. The pass is a gather
+// of 7 scattered values per thread and bound by their latency, so five times
+// the threads, each with a fifth of the registers, is what it needs: mean of
+// a Sedov run's launches on levels 7-9 26.7 -> 14.3 us, on levels 5-6 (a few
+// thousand entries) 5.6 -> 2.1 us, against one thread per entry.
+static __global__ void __launch_bounds__(128) interp_blocks_var_kernel(const double* __restrict__ uold,
+                                                                       const int32_t* __restrict__ cells7,
+                                                                       int32_t nentry, int64_t ncell,
+                                                                       double* __restrict__ out, int itype,
+                                                                       const double* __restrict__ gate) {
+  RB_GATE(gate);
+  const int e = blockIdx.x * 128 + threadIdx.x, v = blockIdx.y;
+  if (e >= nentry) return;
+  const double* u = uold + v * ncell;
+  double a[7], o[8];
+#pragma unroll
+  for (int j = 0; j < 7; j++) a[j] = u[cells7[(int64_t)e * 7 + j]];
+  interp_one_var(a, itype, o);
+  // 64-byte rows: (e * 8) doubles from a 256-byte aligned buffer
+  double2* row = reinterpret_cast<double2*>(out + ((int64_t)v * nentry + e) * 8);
+#pragma unroll
+  for (int k = 0; k < 4; k++) row[k] = make_double2(o[2 * k], o[2 * k + 1]);
+}
+
 // The state of octs created by refinement (make_grid_fine,
 // amr/refine_utils.f90:590-948, through interpol_hydro,
 // hydro/interpol_hydro.f90:268-444): the 8 children of each new oct prolonged
@@ -286,46 +311,43 @@ static __global__ void prolong_new_octs_kernel(double* __restrict__ uold, const 
 // contrib[k] = slot*6 + face (face 0..5 = -x,+x,-y,+y,-z,+z).
 // With pressure_fix (divu non-null) divu and enew get the same corrections
 // from corr_tmp[slot][face][4][2] (godunov_fine.f90:831-856, 883-906).
-static __global__ void apply_corrections_kernel(double* __restrict__ unew, const int32_t* __restrict__ tgt,
-                                         const int32_t* __restrict__ off, const int32_t* __restrict__ contrib,
-                                         int32_t ntgt, const double* __restrict__ corr_flux, int64_t ncell,
-                                         const double* __restrict__ gate, double* __restrict__ divu = nullptr,
-                                         double* __restrict__ enew = nullptr,
-                                         const double* __restrict__ corr_tmp = nullptr) {
+// One thread per (target, value): the contributions of one value are a serial
+// chain of dependent loads, the values of a target are independent, and the
+// lanes of a target read its contributions' fluxes from the same lines (mean
+// of a Sedov run's launches on levels 7-9 16.5 -> 10.9 us, on levels 5-6
+// 5.3 -> 2.9 us, against one thread per target).
+static __global__ void __launch_bounds__(128) apply_corrections_kernel(
+    double* __restrict__ unew, const int32_t* __restrict__ tgt, const int32_t* __restrict__ off,
+    const int32_t* __restrict__ contrib, int32_t ntgt, const double* __restrict__ corr_flux, int64_t ncell,
+    const double* __restrict__ gate, double* __restrict__ divu, double* __restrict__ enew,
+    const double* __restrict__ corr_tmp) {
   RB_GATE(gate);
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nval = divu ? 7 : 5;
+  const int64_t id = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  const int t = (int)(id / nval), v = (int)(id % nval);
   if (t >= ntgt) return;
-  const int64_t dc = tgt[t];
   const double oneontwotondim = 1.0 / 8.0;
-  for (int v = 0; v < 5; v++) {
-    double u = unew[v * ncell + dc];
-    for (int k = off[t]; k < off[t + 1]; k++) {
-      const int slot = contrib[k] / 6, face = contrib[k] % 6;
-      const double* fl = corr_flux + (int64_t)slot * 120 + face * 20;
-      if ((face & 1) == 0) {
-        for (int c = 0; c < 4; c++) u = u - fl[c * 5 + v] * oneontwotondim;
-      } else {
-        for (int c = 0; c < 4; c++) u = u + fl[c * 5 + v] * oneontwotondim;
-      }
-    }
-    unew[v * ncell + dc] = u;
-  }
-  if (divu) {
-    for (int t2 = 0; t2 < 2; t2++) {
-      double* arr = t2 == 0 ? divu : enew;
-      double u = arr[dc];
-      for (int k = off[t]; k < off[t + 1]; k++) {
-        const int slot = contrib[k] / 6, face = contrib[k] % 6;
-        const double* tl = corr_tmp + (int64_t)slot * 48 + face * 8;
-        if ((face & 1) == 0) {
-          for (int c = 0; c < 4; c++) u = u - tl[c * 2 + t2] * oneontwotondim;
-        } else {
-          for (int c = 0; c < 4; c++) u = u + tl[c * 2 + t2] * oneontwotondim;
-        }
-      }
-      arr[dc] = u;
+  double* dst = (v < 5 ? unew + v * ncell : v == 5 ? divu : enew) + tgt[t];
+  // a face's 4 fine cells: stride 5 of [4][5] unew fluxes, stride 2 of [4][2] divu/enew fluxes
+  const double* src = v < 5 ? corr_flux + v : corr_tmp + (v - 5);
+  const int per_face = v < 5 ? 20 : 8, st = v < 5 ? 5 : 2;
+  double u = *dst;
+  const int k1 = off[t + 1];
+  for (int k = off[t]; k < k1; k++) {
+    const int sf = contrib[k];  // slot*6 + face
+    const double* fl = src + (int64_t)sf * per_face;
+    double f[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) f[c] = fl[c * st];
+    if ((sf % 6 & 1) == 0) {
+#pragma unroll
+      for (int c = 0; c < 4; c++) u = u - f[c] * oneontwotondim;
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; c++) u = u + f[c] * oneontwotondim;
     }
   }
+  *dst = u;
 }
 
 // courant_fine (courant_fine.f90:1-159): per-block partial (min dt, mass,

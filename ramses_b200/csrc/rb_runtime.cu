@@ -1281,6 +1281,20 @@ int launch_tile(rb_context* c, int shape, const rb::TileArgs& a, int grid) {
   return RB_OK;
 }
 
+// interpol_hydro of the level's missing neighbour blocks
+int interp_impl(rb_context* c, Level& L, const double* gate) {
+  if (!L.ninterp) return RB_OK;
+  const unsigned nb = (unsigned)((L.ninterp + 127) / 128);
+  if (c->hp.interpol_var == 0)
+    rb::interp_blocks_var_kernel<<<dim3(nb, 5), 128, 0, c->stream>>>(c->d_uold, L.d_interp7, L.ninterp, c->ncell,
+                                                                     L.d_interp_buf, c->hp.interpol_type, gate);
+  else
+    rb::interp_blocks_kernel<<<nb, 128, 0, c->stream>>>(c->d_uold, L.d_interp7, L.ninterp, c->ncell, L.d_interp_buf,
+                                                        c->hp, gate);
+  RB_CUDA(cudaGetLastError());
+  return RB_OK;
+}
+
 // fuse_unew: the level has no finer octs, so at godunov time its unew is
 // set_unew's copy of uold (no fine-to-coarse correction went into it); the
 // kernel then starts the update from uold and writes unew without reading it
@@ -1291,12 +1305,7 @@ int godunov_impl(rb_context* c, int l, double dt, bool timed, const double* dt_d
   if (!L.noct) return RB_OK;
   if (!dt_dev && (!(dt > 0.0) || !std::isfinite(dt)))
     return fail(RB_ERR_INVALID, "dt=%g must be positive and finite", dt);
-  if (L.ninterp) {
-    rb::interp_blocks_kernel<<<(L.ninterp + 127) / 128, 128, 0, c->stream>>>(c->d_uold, L.d_interp7, L.ninterp,
-                                                                             c->ncell, L.d_interp_buf, c->hp,
-                                                                             c->gate);
-    RB_CUDA(cudaGetLastError());
-  }
+  RB_TRY(interp_impl(c, L, c->gate));
   rb::TileArgs a = tile_args(c, L, dt);
   a.dt_dev = dt_dev;
   if (fuse_unew) a.fused = 2;
@@ -1305,7 +1314,8 @@ int godunov_impl(rb_context* c, int l, double dt, bool timed, const double* dt_d
   RB_TRY(launch_tile(c, L.shape, a, L.ntile));
   if (timed) RB_CUDA(cudaEventRecord(c->ev1, c->stream));
   if (L.ntgt) {
-    rb::apply_corrections_kernel<<<(L.ntgt + 127) / 128, 128, 0, c->stream>>>(
+    const int64_t nval = (int64_t)L.ntgt * (c->d_divu ? 7 : 5);
+    rb::apply_corrections_kernel<<<(unsigned)((nval + 127) / 128), 128, 0, c->stream>>>(
         c->d_unew, L.d_tgt, L.d_tgt_off, L.d_contrib, L.ntgt, L.d_corr_flux, c->ncell, c->gate, c->d_divu, c->d_enew,
         L.d_corr_tmp);
     RB_CUDA(cudaGetLastError());
@@ -2126,12 +2136,7 @@ int rb_set_tile_shape(rb_context* c, int l, int shape) {
     if (smem > 227 * 1024 || !shape_fits(c, l, s)) continue;
     L.shape = s;
     RB_TRY(build_level_tables(c, l, c->idx));
-    if (L.ninterp) {
-      rb::interp_blocks_kernel<<<(L.ninterp + 127) / 128, 128, 0, c->stream>>>(c->d_uold, L.d_interp7, L.ninterp,
-                                                                               c->ncell, L.d_interp_buf, c->hp,
-                                                                               nullptr);
-      RB_CUDA(cudaGetLastError());
-    }
+    RB_TRY(interp_impl(c, L, nullptr));
     RB_CUDA(cudaMemcpyAsync(c->d_stage, keep_unew, (size_t)c->ncell * 5 * sizeof(double), cudaMemcpyDeviceToDevice,
                             c->stream));
     c->d_unew = c->d_stage;
