@@ -120,18 +120,21 @@ __device__ __forceinline__ void pf_fix_cell(double u[5], double divu, double ene
   if (e_cons < e_trunc) u[4] = enew + e_kin;
 }
 
-// pressure_fix part of set_unew (godunov_fine.f90:71-86): divu = 0 and enew
-// = the internal energy of uold, for every cell of the active octs.
-static __global__ void pf_set_unew_kernel(const double* __restrict__ uold, double* __restrict__ divu,
-                                          double* __restrict__ enew, const int32_t* __restrict__ active,
-                                          int32_t noct, int64_t ncell, int32_t ncoarse, double smallr,
-                                          const double* __restrict__ gate) {
+// set_unew with pressure_fix (godunov_fine.f90:71-86): unew = uold, divu = 0
+// and enew = the internal energy of uold, for every cell of the active octs.
+static __global__ void pf_set_unew_kernel(const double* __restrict__ uold, double* __restrict__ unew,
+                                          double* __restrict__ divu, double* __restrict__ enew,
+                                          const int32_t* __restrict__ active, int32_t noct, int64_t ncell,
+                                          int32_t ncoarse, double smallr, const double* __restrict__ gate) {
   RB_GATE(gate);
   const int64_t n = (int64_t)noct * 8;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t dc = ncoarse + (int64_t)active[i >> 3] * 8 + (i & 7);
     double u[5];
+#pragma unroll
     for (int v = 0; v < 5; v++) u[v] = uold[v * ncell + dc];
+#pragma unroll
+    for (int v = 0; v < 5; v++) unew[v * ncell + dc] = u[v];
     divu[dc] = 0.0;
     enew[dc] = pf_eint(u, smallr);
   }
@@ -472,78 +475,152 @@ static __global__ void __launch_bounds__(RB_RED_NT) reduce_partials_kernel(const
 // ---- device-resident amr_step clock ----------------------------------------
 // The scalar bookkeeping of amr_step (amr/amr_step.f90:320-331,571-576),
 // newdt_fine (pm/newdt_fine.f90:47-51,173) and update_time's t/nstep advance
-// (amr/update_time.f90:330-331) runs in single-thread kernels on one array
-// `s`, so a sequence of coarse steps needs no host round trip and can be
-// captured into a CUDA graph. Every level kernel of a coarse step takes
-// gate = s + RB_S_DONE and returns at once when the run is over (t >= t_end or
-// the requested number of coarse steps done), so a graph of K coarse steps
-// stops exactly where a host loop would.
+// (amr/update_time.f90:330-331) lives in one array `s`, so a sequence of
+// coarse steps needs no host round trip and can be captured into a CUDA
+// graph. Every level kernel of a coarse step takes gate = s + RB_S_DONE and
+// returns at once when the run is over (t >= t_end or the requested number of
+// coarse steps done), so a graph of K coarse steps stops exactly where a host
+// loop would.
+//
+// Between two godunov passes the bookkeeping is a short list of scalar
+// operations. The list is executed by the last CTA of the pass that completes
+// the level step (set_uold + restriction, or the finest level's CFL pass),
+// which also holds the level's next CFL condition: the state that
+// courant_fine(l) reads at the start of an amr_step(l) is the state that the
+// previous step of level l left (only that step's set_uold and upload_fine
+// write the level's cells), so its wave speeds are taken in the pass that
+// writes it. On a small octree (levels 4-6, 70 launches per coarse step, 2-10
+// us each, mostly launch latency) this and the merged set_unew leave 19:
+// 3.03 -> 2.30 ms per 12 steps; on levels 6-9 (4 M leaf cells), where the
+// passes saved are memory traffic, 113.0 -> 104.4 ms per 16 steps.
 #define RB_NLV (RB_MAXLEVEL + 2)
 #define RB_S_DTNEW 0
 #define RB_S_DTOLD RB_NLV
-#define RB_S_T (2 * RB_NLV)
-#define RB_S_NSTEP (2 * RB_NLV + 1)
-#define RB_S_MASS (2 * RB_NLV + 2)
-#define RB_S_EKIN (2 * RB_NLV + 3)
-#define RB_S_EINT (2 * RB_NLV + 4)
-#define RB_S_DONE (2 * RB_NLV + 5)
-#define RB_S_TEND (2 * RB_NLV + 6)
-#define RB_S_MAXC (2 * RB_NLV + 7)
-#define RB_S_COARSE (2 * RB_NLV + 8)
-#define RB_S_SIZE (2 * RB_NLV + 16)
+#define RB_S_DTLEV (2 * RB_NLV)      // CFL dt of the level's current state (1e300: no leaf cell)
+#define RB_S_DTCMP (3 * RB_NLV)      // courant_factor*dx/smallc of the level, or boxlen/smallc without leaf cells
+#define RB_S_NSUB (4 * RB_NLV)       // nsubcycle of the level
+#define RB_S_T (5 * RB_NLV)
+#define RB_S_NSTEP (5 * RB_NLV + 1)
+#define RB_S_DTMAX (5 * RB_NLV + 2)  // boxlen/smallc
+#define RB_S_LMIN (5 * RB_NLV + 3)
+#define RB_S_DONE (5 * RB_NLV + 4)
+#define RB_S_TEND (5 * RB_NLV + 5)
+#define RB_S_MAXC (5 * RB_NLV + 6)
+#define RB_S_COARSE (5 * RB_NLV + 7)
+#define RB_S_SIZE (5 * RB_NLV + 8)
 
-// start of a coarse step: decide whether it runs; reset the level totals
-static __global__ void sched_gate_kernel(double* __restrict__ s) {
-  const bool done = !(s[RB_S_T] < s[RB_S_TEND]) || !(s[RB_S_COARSE] < s[RB_S_MAXC]);
-  s[RB_S_DONE] = done ? 1.0 : 0.0;
-  if (!done) s[RB_S_MASS] = s[RB_S_EKIN] = s[RB_S_EINT] = 0.0;
-}
-
-// newdt_fine + courant_fine of level l from the level's CFL partials:
-// dtold(l)=dtnew(l); dtnew(l)=min(boxlen/smallc, courant); for l>levelmin
-// dtnew(l)=min(dtnew(l-1)/nsubcycle(l-1), dtnew(l)); level totals accumulated.
-static __global__ void __launch_bounds__(RB_RED_NT) sched_courant_kernel(const double* __restrict__ partial, int n, int l,
-                                                                  int levelmin, double dt_cmpdt0, int any_leaf,
-                                                                  double dt_max, double nsub_prev,
-                                                                  double* __restrict__ s) {
-  if (s[RB_S_DONE] != 0.0) return;
-  __shared__ double red[4][RB_RED_NT];
-  reduce4_block(partial, n, red);
-  if (threadIdx.x == 0) {
-    s[RB_S_DTOLD + l] = s[RB_S_DTNEW + l];
-    const double dt_lev = fmn(dt_cmpdt0, red[0][0]);
-    const double dt_all = any_leaf ? fmn(dt_max, dt_lev) : dt_max;
-    s[RB_S_MASS] = s[RB_S_MASS] + red[1][0];
-    s[RB_S_EKIN] = s[RB_S_EKIN] + red[2][0];
-    s[RB_S_EINT] = s[RB_S_EINT] + red[3][0];
-    double dtn = fmn(dt_max, dt_all);
-    if (l > levelmin) dtn = fmn(s[RB_S_DTNEW + l - 1] / nsub_prev, dtn);
-    s[RB_S_DTNEW + l] = dtn;
+// Scalar operations, code = op << 8 | level:
+//  GATE     start of a coarse step: raise the done flag if the run is over
+//           (the operations after it are skipped then)
+//  COURANT  newdt_fine + courant_fine: dtold(l) = dtnew(l), dtnew(l) =
+//           min(boxlen/smallc, CFL dt), for l > levelmin also bounded by
+//           dtnew(l-1)/nsubcycle(l-1)
+//  ADVANCE  level l was the finest of the step: t, nstep. ADVANCE1: level l+1
+//           exists without octs, its dtold and dtnew follow
+//  END1     end of amr_step(l), nsubcycle(l-1) == 1: dtnew(l-1) = dtnew(l)
+//  END2     end of the second subcycle: dtnew(l-1) = dtold(l) + dtnew(l)
+//  FINISH   one coarse step done
+enum { RB_OP_GATE = 0, RB_OP_COURANT, RB_OP_ADVANCE, RB_OP_ADVANCE1, RB_OP_END1, RB_OP_END2, RB_OP_FINISH };
+#define RB_PROG_MAX 112  // COURANT and two ENDs for every level, and the rest
+struct SchedProg {
+  int32_t n;
+  uint16_t op[RB_PROG_MAX];
+};
+__device__ inline void sched_run(double* __restrict__ s, const SchedProg& p) {
+  for (int i = 0; i < p.n; i++) {
+    const int l = p.op[i] & 0xff;
+    switch (p.op[i] >> 8) {
+      case RB_OP_GATE:
+        if (!(s[RB_S_T] < s[RB_S_TEND]) || !(s[RB_S_COARSE] < s[RB_S_MAXC])) {
+          s[RB_S_DONE] = 1.0;
+          return;
+        }
+        break;
+      case RB_OP_COURANT: {
+        s[RB_S_DTOLD + l] = s[RB_S_DTNEW + l];
+        double dt = fmn(s[RB_S_DTMAX], fmn(s[RB_S_DTCMP + l], s[RB_S_DTLEV + l]));
+        if (l > (int)s[RB_S_LMIN]) dt = fmn(s[RB_S_DTNEW + l - 1] / s[RB_S_NSUB + l - 1], dt);
+        s[RB_S_DTNEW + l] = dt;
+        break;
+      }
+      case RB_OP_ADVANCE1:
+        s[RB_S_DTOLD + l + 1] = s[RB_S_DTNEW + l] / s[RB_S_NSUB + l];
+        s[RB_S_DTNEW + l + 1] = s[RB_S_DTNEW + l] / s[RB_S_NSUB + l];
+        // fall through
+      case RB_OP_ADVANCE:
+        s[RB_S_T] = s[RB_S_T] + s[RB_S_DTNEW + l];
+        s[RB_S_NSTEP] = s[RB_S_NSTEP] + 1.0;
+        break;
+      case RB_OP_END1: s[RB_S_DTNEW + l - 1] = s[RB_S_DTNEW + l]; break;
+      case RB_OP_END2: s[RB_S_DTNEW + l - 1] = s[RB_S_DTOLD + l] + s[RB_S_DTNEW + l]; break;
+      case RB_OP_FINISH: s[RB_S_COARSE] = s[RB_S_COARSE] + 1.0; break;
+    }
   }
 }
+static __global__ void sched_kernel(double* __restrict__ s, const SchedProg p) {
+  if (s[RB_S_DONE] == 0.0) sched_run(s, p);
+}
 
-// the finest level of this step is l: advance t and nstep; when the next
-// level exists but holds no oct (mode 1) also set its dtold/dtnew
-static __global__ void sched_advance_kernel(double* __restrict__ s, int l, int mode, double nsub_l) {
-  if (s[RB_S_DONE] != 0.0) return;
-  if (mode == 1) {
-    s[RB_S_DTOLD + l + 1] = s[RB_S_DTNEW + l] / nsub_l;
-    s[RB_S_DTNEW + l + 1] = s[RB_S_DTNEW + l] / nsub_l;
+// What the last CTA of a level pass does with the level's largest wave speed.
+struct CflTail {
+  unsigned long long* smax;  // bit pattern of the largest speed so far (zero between passes)
+  unsigned* count;           // CTAs done (zero between passes)
+  double* s;                 // the clock; null: the pass has no tail
+  double dx, courant_factor;
+  int32_t l;
+  SchedProg prog;
+};
+// Every thread of every CTA of the pass calls this with its own largest
+// speed (>= 0, which orders like its bit pattern; the maximum does not depend
+// on the order of the CTAs).
+template <int NT>
+__device__ __forceinline__ void cfl_tail(double smax, const CflTail& t) {
+  __shared__ double red[NT / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) smax = fmx(smax, __shfl_xor_sync(0xffffffffu, smax, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = smax;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < NT / 32; w++) smax = fmx(smax, red[w]);
+  if (smax > 0.0) atomicMax(t.smax, (unsigned long long)__double_as_longlong(smax));
+  __threadfence();
+  if (atomicAdd(t.count, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  const double m = __longlong_as_double((long long)atomicExch(t.smax, 0ull));
+  *t.count = 0u;
+  t.s[RB_S_DTLEV + t.l] = m > 0.0 ? cfl_dt_from_speed(m, t.dx, t.courant_factor) : 1.0e300;
+  sched_run(t.s, t.prog);
+}
+
+// The CFL condition of level l's leaf cells in state u: before a run's first
+// step (with unew non-null also set_unew, unew = u), and after each step of a
+// finest level, whose state needs no set_uold pass (see amr_step_dev).
+// FAST (FP32-mixed contexts): the wave speed of cfl_speed_fast.
+template <int NT, bool FAST>
+static __global__ void __launch_bounds__(NT) level_cfl_kernel(const double* __restrict__ u,
+                                                              const int32_t* __restrict__ son,
+                                                              const int32_t* __restrict__ active, int32_t noct,
+                                                              int64_t ncell, int32_t ncoarse, rb_hydro_params hp,
+                                                              double* __restrict__ unew,
+                                                              const double* __restrict__ gate,
+                                                              const __grid_constant__ CflTail tail) {
+  RB_GATE(gate);
+  double smax = 0.0;
+  const int64_t n = (int64_t)noct * 8;
+  for (int64_t i = blockIdx.x * (int64_t)NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT) {
+    const int64_t dc = ncoarse + (int64_t)active[i >> 3] * 8 + (i & 7);
+    const bool leaf = son[dc] == 0;
+    if (!leaf && !unew) continue;
+    double q[5];
+#pragma unroll
+    for (int v = 0; v < 5; v++) q[v] = u[v * ncell + dc];
+    if (unew) {
+#pragma unroll
+      for (int v = 0; v < 5; v++) unew[v * ncell + dc] = q[v];
+    }
+    if (leaf) smax = fmx(smax, FAST ? cfl_speed_fast(q, hp) : cfl_speed(q, hp));
   }
-  s[RB_S_T] = s[RB_S_T] + s[RB_S_DTNEW + l];
-  s[RB_S_NSTEP] = s[RB_S_NSTEP] + 1.0;
-}
-
-// end of amr_step(l, icount) for l > levelmin (amr_step.f90:571-576)
-static __global__ void sched_end_kernel(double* __restrict__ s, int l, int nsub_prev_is_one, int icount) {
-  if (s[RB_S_DONE] != 0.0) return;
-  if (nsub_prev_is_one) s[RB_S_DTNEW + l - 1] = s[RB_S_DTNEW + l];
-  if (icount == 2) s[RB_S_DTNEW + l - 1] = s[RB_S_DTOLD + l] + s[RB_S_DTNEW + l];
-}
-
-static __global__ void sched_finish_kernel(double* __restrict__ s) {
-  if (s[RB_S_DONE] != 0.0) return;
-  s[RB_S_COARSE] = s[RB_S_COARSE] + 1.0;
+  cfl_tail<NT>(smax, tail);
 }
 
 // hydro_refine (godunov_utils.f90:125-263) for one cell along one direction:
@@ -694,21 +771,31 @@ static __global__ void upload_fine_kernel(double* __restrict__ uold, const int32
 // pressure_fix (divu non-null) the copied cells get set_uold's energy fix
 // (dt: *dt_dev if non-null, else dt_val); the split cells' fix would be
 // overwritten by the restriction.
-static __global__ void set_uold_upload_kernel(double* __restrict__ uold, const double* __restrict__ unew,
-                                              const int32_t* __restrict__ son, const int32_t* __restrict__ active,
-                                              int32_t noct, int64_t ncell, int32_t ncoarse, rb_hydro_params hp,
-                                              int do_upload, const double* __restrict__ gate,
-                                              const double* __restrict__ divu = nullptr,
-                                              const double* __restrict__ enew = nullptr, double dx = 0.0,
-                                              const double* __restrict__ dt_dev = nullptr, double dt_val = 0.0) {
+// In a device-scheduled run (tail.s non-null) the pass also takes the leaf
+// cells' wave speeds for the level's next CFL condition, and with next_unew
+// set it does the set_unew of the level's next step: unew = uold, which for
+// the copied cells holds already.
+template <int NT, bool FAST>
+static __global__ void __launch_bounds__(NT) set_uold_upload_kernel(
+    double* __restrict__ uold, double* __restrict__ unew, const int32_t* __restrict__ son,
+    const int32_t* __restrict__ active, int32_t noct, int64_t ncell, int32_t ncoarse, rb_hydro_params hp,
+    int do_upload, const double* __restrict__ gate, const double* __restrict__ divu, const double* __restrict__ enew,
+    double dx, const double* __restrict__ dt_dev, double dt_val, int next_unew,
+    const __grid_constant__ CflTail tail) {
   RB_GATE(gate);
   const double dt = dt_dev ? *dt_dev : dt_val;
+  const bool cfl = tail.s != nullptr;
+  double smax = 0.0;
   const int64_t n = (int64_t)noct * 8;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t i = blockIdx.x * (int64_t)NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT) {
     const int64_t dc = ncoarse + (int64_t)active[i >> 3] * 8 + (i & 7);
     const int gs = do_upload ? son[dc] : 0;
     if (gs > 0) {
       restrict_cell(uold, dc, gs, ncell, ncoarse, hp);
+      if (next_unew) {
+#pragma unroll
+        for (int v = 0; v < 5; v++) unew[v * ncell + dc] = uold[v * ncell + dc];
+      }
     } else {
       double u[5];
 #pragma unroll
@@ -716,8 +803,10 @@ static __global__ void set_uold_upload_kernel(double* __restrict__ uold, const d
       if (divu) pf_fix_cell(u, divu[dc], enew[dc], dx, dt, hp.smallr, hp.beta_fix);
 #pragma unroll
       for (int v = 0; v < 5; v++) uold[v * ncell + dc] = u[v];
+      if (cfl) smax = fmx(smax, FAST ? cfl_speed_fast(u, hp) : cfl_speed(u, hp));
     }
   }
+  if (cfl) cfl_tail<NT>(smax, tail);
 }
 
 // ---------------------------------------------------------------------------

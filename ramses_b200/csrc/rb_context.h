@@ -165,6 +165,7 @@ struct rb_context {
   double* h_red = nullptr;          // pinned [8]
   double* d_sched = nullptr;        // [RB_S_SIZE] device-resident amr_step clock
   double* h_sched = nullptr;        // pinned [RB_S_SIZE]
+  unsigned long long* d_cfl = nullptr;  // [2] largest wave speed and CTA count of the level pass under way (CflTail)
   uint8_t* d_flag = nullptr;        // hydro_flag output, one byte per cell of a level
   int64_t flag_cap = 0;
   const double* gate = nullptr;     // level kernels return early when *gate != 0

@@ -1069,14 +1069,14 @@ int check_level(rb_context* c, int l) {
 int set_unew_impl(rb_context* c, int l) {
   Level& L = c->lv[l];
   if (!L.noct) return RB_OK;
-  rb::copy_octs_kernel<<<grid_for((int64_t)L.noct * 8, 256), 256, 0, c->stream>>>(
-      c->d_uold, c->d_unew, L.d_active, L.noct, c->ncell, c->mp.ncoarse, c->gate);
+  const int grid = grid_for((int64_t)L.noct * 8, 256);
+  if (c->hp.pressure_fix)
+    rb::pf_set_unew_kernel<<<grid, 256, 0, c->stream>>>(c->d_uold, c->d_unew, c->d_divu, c->d_enew, L.d_active, L.noct,
+                                                        c->ncell, c->mp.ncoarse, c->hp.smallr, c->gate);
+  else
+    rb::copy_octs_kernel<<<grid, 256, 0, c->stream>>>(c->d_uold, c->d_unew, L.d_active, L.noct, c->ncell,
+                                                      c->mp.ncoarse, c->gate);
   RB_CUDA(cudaGetLastError());
-  if (c->hp.pressure_fix) {
-    rb::pf_set_unew_kernel<<<grid_for((int64_t)L.noct * 8, 256), 256, 0, c->stream>>>(
-        c->d_uold, c->d_divu, c->d_enew, L.d_active, L.noct, c->ncell, c->mp.ncoarse, c->hp.smallr, c->gate);
-    RB_CUDA(cudaGetLastError());
-  }
   return RB_OK;
 }
 
@@ -1118,15 +1118,20 @@ int set_uold_impl(rb_context* c, int l) {
 
 // set_uold + upload_fine of level l in one pass (set_uold_upload_kernel);
 // with pressure_fix, the pdV term before, and the energy fix in the same
-// pass. dt: *dt_dev if non-null.
-int set_uold_upload_impl(rb_context* c, int l, const double* dt_dev, double dt) {
+// pass. dt: *dt_dev if non-null. tail, next_unew: see the kernel.
+int set_uold_upload_impl(rb_context* c, int l, const double* dt_dev, double dt, const rb::CflTail* tail = nullptr,
+                         int next_unew = 0) {
   Level& L = c->lv[l];
   if (!L.noct) return RB_OK;
   const int do_upload = (l < c->mp.nlevelmax && L.has_refined) ? 1 : 0;
   if (c->hp.pressure_fix) RB_TRY(pdv_impl(c, l, dt_dev, dt));
-  rb::set_uold_upload_kernel<<<grid_for((int64_t)L.noct * 8, 256), 256, 0, c->stream>>>(
+  rb::CflTail none;
+  memset(&none, 0, sizeof none);
+  auto k = c->precision == RB_PREC_MIXED ? rb::set_uold_upload_kernel<256, true> : rb::set_uold_upload_kernel<256, false>;
+  // with a tail: one wave of CTAs, each of which signals its completion once
+  k<<<grid_for((int64_t)L.noct * 8, 256, tail ? 148 * 8 : 148 * 32), 256, 0, c->stream>>>(
       c->d_uold, c->d_unew, c->d_son, L.d_active, L.noct, c->ncell, c->mp.ncoarse, c->hp, do_upload, c->gate,
-      c->d_divu, c->d_enew, L.dx, dt_dev, dt);
+      c->d_divu, c->d_enew, L.dx, dt_dev, dt, next_unew, tail ? *tail : none);
   RB_CUDA(cudaGetLastError());
   return RB_OK;
 }
@@ -1299,15 +1304,22 @@ int interp_impl(rb_context* c, Level& L, const double* gate) {
 // set_unew's copy of uold (no fine-to-coarse correction went into it); the
 // kernel then starts the update from uold and writes unew without reading it
 // (the caller skips set_unew's copy for the level). Same values bit for bit.
+// swapped (with fuse_unew): the level's state is in unew and the new one goes
+// to uold. with_interp: 0 where the level's prolongation entries already hold
+// the values of this step.
 int godunov_impl(rb_context* c, int l, double dt, bool timed, const double* dt_dev = nullptr,
-                 bool fuse_unew = false) {
+                 bool fuse_unew = false, bool swapped = false, bool with_interp = true) {
   Level& L = c->lv[l];
   if (!L.noct) return RB_OK;
   if (!dt_dev && (!(dt > 0.0) || !std::isfinite(dt)))
     return fail(RB_ERR_INVALID, "dt=%g must be positive and finite", dt);
-  RB_TRY(interp_impl(c, L, c->gate));
+  if (with_interp) RB_TRY(interp_impl(c, L, c->gate));
   rb::TileArgs a = tile_args(c, L, dt);
   a.dt_dev = dt_dev;
+  if (swapped) {
+    a.uold = c->d_unew;
+    a.unew = c->d_uold;
+  }
   if (fuse_unew) a.fused = 2;
   if (!dt_dev) c->dt_godunov[l] = dt;
   if (timed) RB_CUDA(cudaEventRecord(c->ev0, c->stream));
@@ -1392,56 +1404,134 @@ int amr_step_impl(rb_context* c, int l, int icount) {
 }
 
 // ---- device-scheduled coarse steps ----------------------------------------
-// Twin of amr_step_impl with the same launches, in the same order, on the same
-// stream; the scalar scheduler state lives in c->d_sched (sched_* kernels)
-// and every level kernel is gated on c->d_sched[RB_S_DONE].
-int courant_blocks(const rb_context* c, int l) { return grid_for((int64_t)c->lv[l].noct * 8, 256, 148 * 8); }
+// Twin of amr_step_impl on the same stream; the scalar scheduler state lives
+// in c->d_sched, the scalar operations run in the tails of the level passes
+// (sched_run), and every level kernel is gated on c->d_sched[RB_S_DONE].
 
-int amr_step_dev(rb_context* c, int l, int icount) {
+// A coarse step as the sequence of its level steps (l, icount), each with the
+// scalar operations that follow it up to the next level step; lead: those
+// before the first one. ADVANCE only reads dtnew(l), which nothing between
+// the finest level's courant_fine and the end of its step changes, so it
+// follows that step (t then never runs ahead of the state).
+struct LevelStep {
+  int l, icount;
+  std::vector<uint16_t> ops;
+};
+struct CoarsePlan {
+  std::vector<uint16_t> lead;
+  std::vector<LevelStep> steps;
+};
+void plan_level(const rb_context* c, int l, int icount, CoarsePlan& p) {
+  if (c->lv[l].noct == 0) return;
+  auto op = [&](int code, int lev) {
+    (p.steps.empty() ? p.lead : p.steps.back().ops).push_back((uint16_t)(code << 8 | lev));
+  };
+  op(rb::RB_OP_COURANT, l);
+  const bool finer = l < c->mp.nlevelmax && c->lv[l + 1].noct > 0;
+  if (finer) {
+    plan_level(c, l + 1, 1, p);
+    if (c->mp.nsubcycle[l] == 2) plan_level(c, l + 1, 2, p);
+  }
+  p.steps.push_back({l, icount, {}});
+  if (!finer) op(l < c->mp.nlevelmax ? rb::RB_OP_ADVANCE1 : rb::RB_OP_ADVANCE, l);
+  if (l > c->mp.levelmin) {
+    if (c->mp.nsubcycle[l - 1] == 1) op(rb::RB_OP_END1, l);
+    if (icount == 2) op(rb::RB_OP_END2, l);
+  }
+}
+CoarsePlan plan_coarse(const rb_context* c) {
+  CoarsePlan p;
+  p.lead.push_back(rb::RB_OP_GATE << 8);
+  plan_level(c, c->mp.levelmin, 1, p);
+  if (!p.steps.empty()) {  // the next coarse step's lead follows the last level step
+    auto& ops = p.steps.back().ops;
+    ops.push_back(rb::RB_OP_FINISH << 8);
+    ops.insert(ops.end(), p.lead.begin(), p.lead.end());
+  }
+  return p;
+}
+int make_prog(const std::vector<uint16_t>& ops, rb::SchedProg* p) {
+  if (ops.size() > RB_PROG_MAX) return fail(RB_ERR_CAPACITY, "scheduler program of %zu operations", ops.size());
+  memset(p, 0, sizeof *p);
+  p->n = (int32_t)ops.size();
+  std::copy(ops.begin(), ops.end(), p->op);
+  return RB_OK;
+}
+int make_tail(rb_context* c, int l, const std::vector<uint16_t>& ops, rb::CflTail* t) {
+  memset(t, 0, sizeof *t);
+  t->smax = c->d_cfl;
+  t->count = (unsigned*)(c->d_cfl + 1);
+  t->s = c->d_sched;
+  t->dx = c->lv[l].dx;
+  t->courant_factor = c->hp.courant_factor;
+  t->l = l;
+  return make_prog(ops, &t->prog);
+}
+int sched_impl(rb_context* c, const std::vector<uint16_t>& ops) {
+  rb::SchedProg p;
+  RB_TRY(make_prog(ops, &p));
+  rb::sched_kernel<<<1, 1, 0, c->stream>>>(c->d_sched, p);
+  RB_CUDA(cudaGetLastError());
+  return RB_OK;
+}
+int level_cfl_impl(rb_context* c, int l, const double* u, double* unew, const rb::CflTail& tail) {
   Level& L = c->lv[l];
-  if (L.noct == 0) return RB_OK;
-  double* s = c->d_sched;
-  const int nblk = courant_blocks(c, l);
-  auto k = c->precision == RB_PREC_MIXED ? rb::courant_partial_kernel<256, true> : rb::courant_partial_kernel<256, false>;
-  // + set_unew, which a level without finer octs gets in its godunov kernel
-  const bool fuse = !L.has_refined;
-  k<<<nblk, 256, 0, c->stream>>>(c->d_uold, c->d_son, L.d_active, L.noct, c->ncell, c->mp.ncoarse, L.dx, c->hp,
-                                 c->d_partial, c->gate, fuse ? nullptr : c->d_unew, fuse ? nullptr : c->d_divu,
-                                 fuse ? nullptr : c->d_enew);
+  auto k = c->precision == RB_PREC_MIXED ? rb::level_cfl_kernel<256, true> : rb::level_cfl_kernel<256, false>;
+  k<<<grid_for((int64_t)L.noct * 8, 256, 148 * 8), 256, 0, c->stream>>>(u, c->d_son, L.d_active, L.noct, c->ncell,
+                                                                       c->mp.ncoarse, c->hp, unew, c->gate, tail);
   RB_CUDA(cudaGetLastError());
-  const double nsub_prev = l > c->mp.levelmin ? (double)(float)c->mp.nsubcycle[l - 1] : 1.0;
-  rb::sched_courant_kernel<<<1, RB_RED_NT, 0, c->stream>>>(
-      c->d_partial, nblk, l, c->mp.levelmin, c->hp.courant_factor * L.dx / c->hp.smallc, L.leaf_cells > 0 ? 1 : 0,
-      c->mp.boxlen / c->hp.smallc, nsub_prev, s);
-  RB_CUDA(cudaGetLastError());
-  if (l < c->mp.nlevelmax) {
-    if (c->lv[l + 1].noct > 0) {
-      RB_TRY(amr_step_dev(c, l + 1, 1));
-      if (c->mp.nsubcycle[l] == 2) RB_TRY(amr_step_dev(c, l + 1, 2));
-    } else {
-      rb::sched_advance_kernel<<<1, 1, 0, c->stream>>>(s, l, 1, (double)c->mp.nsubcycle[l]);
-    }
-  } else {
-    rb::sched_advance_kernel<<<1, 1, 0, c->stream>>>(s, l, 2, 1.0);
-  }
-  RB_CUDA(cudaGetLastError());
-  RB_TRY(godunov_impl(c, l, 0.0, false, s + RB_S_DTNEW + l, fuse));
-  RB_TRY(set_uold_upload_impl(c, l, s + RB_S_DTNEW + l, 0.0));
-  RB_TRY(boundary_impl(c, l));
-  if (l > c->mp.levelmin && (c->mp.nsubcycle[l - 1] == 1 || icount == 2)) {
-    rb::sched_end_kernel<<<1, 1, 0, c->stream>>>(s, l, c->mp.nsubcycle[l - 1] == 1 ? 1 : 0, icount);
-    RB_CUDA(cudaGetLastError());
-  }
   return RB_OK;
 }
 
+// The finest level's two subcycles alternate between uold and unew instead of
+// copying unew back: nothing but the level's own godunov pass reads its cells
+// between them (the next coarser level's restriction follows the second one,
+// after which the state is in uold again; a level without finer octs is no
+// father of a prolongation). Not with boundary octs on the level, which are
+// refilled in uold, nor with pressure_fix, whose pdV term reads the old state
+// after the update.
+bool finest_alternates(const rb_context* c, int l) {
+  const Level& L = c->lv[l];
+  return !L.has_refined && l > c->mp.levelmin && c->mp.nsubcycle[l - 1] == 2 && !c->hp.pressure_fix &&
+         (c->btype.empty() || L.h_boff.empty() || L.h_boff.back() == 0);
+}
+
+int level_step_dev(rb_context* c, const LevelStep& st) {
+  const int l = st.l;
+  Level& L = c->lv[l];
+  const double* dt = c->d_sched + RB_S_DTNEW + l;
+  const bool fuse = !L.has_refined;  // set_unew inside the godunov kernel
+  const bool alt = finest_alternates(c, l);
+  // the operations may end the run (GATE), so they follow the boundary fill
+  // where the level has boundary octs
+  const bool bounded = !c->btype.empty() && !L.h_boff.empty() && L.h_boff.back() > 0;
+  rb::CflTail tail;
+  RB_TRY(make_tail(c, l, bounded ? std::vector<uint16_t>() : st.ops, &tail));
+  // the prolongation reads the coarser levels only, which do not change
+  // between the two subcycles of the level: one pass serves both
+  RB_TRY(godunov_impl(c, l, 0.0, false, dt, fuse, alt && st.icount == 2, st.icount != 2));
+  if (alt) return level_cfl_impl(c, l, st.icount == 2 ? c->d_uold : c->d_unew, nullptr, tail);
+  RB_TRY(set_uold_upload_impl(c, l, dt, 0.0, &tail, fuse || c->hp.pressure_fix ? 0 : 1));
+  if (!bounded) return RB_OK;
+  RB_TRY(boundary_impl(c, l));
+  return sched_impl(c, st.ops);
+}
+
 int coarse_step_dev(rb_context* c) {
-  rb::sched_gate_kernel<<<1, 1, 0, c->stream>>>(c->d_sched);
-  RB_CUDA(cudaGetLastError());
-  RB_TRY(amr_step_dev(c, c->mp.levelmin, 1));
-  for (int l = c->mp.levelmin - 1; l >= 1; l--) RB_TRY(upload_fine_impl(c, l));
-  rb::sched_finish_kernel<<<1, 1, 0, c->stream>>>(c->d_sched);
-  RB_CUDA(cudaGetLastError());
+  const CoarsePlan plan = plan_coarse(c);
+  // with pressure_fix, set_unew (with divu and enew) runs where amr_step has
+  // it, at the start of each step of a level with finer octs
+  std::vector<char> unew_due(RB_MAXLEVEL + 2, 1);
+  for (const LevelStep& st : plan.steps) {
+    if (c->hp.pressure_fix)
+      for (int l = c->mp.levelmin; l < st.l; l++)
+        if (unew_due[l] && c->lv[l].has_refined) {
+          RB_TRY(set_unew_impl(c, l));
+          unew_due[l] = 0;
+        }
+    RB_TRY(level_step_dev(c, st));
+    unew_due[st.l] = 1;
+  }
   return RB_OK;
 }
 
@@ -1490,6 +1580,14 @@ int sched_upload(rb_context* c, int64_t max_coarse, double t_end) {
     h[RB_S_DTNEW + l] = c->dtnew[l];
     h[RB_S_DTOLD + l] = c->dtold[l];
   }
+  const double dt_max = c->mp.boxlen / c->hp.smallc;
+  for (int l = 1; l <= c->mp.nlevelmax; l++) {
+    h[RB_S_DTLEV + l] = 1.0e300;
+    h[RB_S_DTCMP + l] = c->lv[l].leaf_cells > 0 ? c->hp.courant_factor * c->lv[l].dx / c->hp.smallc : dt_max;
+    h[RB_S_NSUB + l] = (double)(float)c->mp.nsubcycle[l];
+  }
+  h[RB_S_DTMAX] = dt_max;
+  h[RB_S_LMIN] = (double)c->mp.levelmin;
   h[RB_S_T] = c->t;
   h[RB_S_NSTEP] = (double)c->nstep;
   h[RB_S_TEND] = t_end;
@@ -1509,9 +1607,6 @@ int sched_download(rb_context* c, int64_t* coarse_out) {
   }
   c->t = h[RB_S_T];
   c->nstep = (int64_t)h[RB_S_NSTEP];
-  c->mass_tot = h[RB_S_MASS];
-  c->ekin_tot = h[RB_S_EKIN];
-  c->eint_tot = h[RB_S_EINT];
   if (coarse_out) *coarse_out = (int64_t)h[RB_S_COARSE];
   return RB_OK;
 }
@@ -1522,19 +1617,27 @@ int sched_download(rb_context* c, int64_t* coarse_out) {
 int run_async_begin(rb_context* c, double t_end, int64_t max_coarse) {
   RB_TRY(sync_oct(c));
   oct_changed(c);
-  int nblk = 1;
-  for (int l = 1; l <= c->mp.nlevelmax; l++)
-    if (c->lv[l].noct) nblk = std::max(nblk, courant_blocks(c, l));
-  RB_TRY(ensure_partial(c, nblk));
   RB_TRY(sched_upload(c, max_coarse, t_end));
   c->gate = c->d_sched + RB_S_DONE;
-  return RB_OK;
+  // the starting state's CFL condition on every level (with set_unew where
+  // the level steps do it ahead), then the first step's scalar operations
+  for (int l = c->mp.levelmin; l <= c->mp.nlevelmax && c->lv[l].noct; l++) {
+    rb::CflTail tail;
+    RB_TRY(make_tail(c, l, {}, &tail));
+    RB_TRY(level_cfl_impl(c, l, c->d_uold, c->lv[l].has_refined && !c->hp.pressure_fix ? c->d_unew : nullptr, tail));
+  }
+  return sched_impl(c, plan_coarse(c).lead);
 }
 
 int run_async_chunk(rb_context* c, int chunk, bool use_graph) { return enqueue_chunk(c, chunk, use_graph); }
 
 int run_async_end(rb_context* c, int64_t* coarse_out) {
   c->gate = nullptr;
+  // the levels below levelmin are read by no step: one restriction of the
+  // final state (adaptive_loop.f90:118-205 restricts after every coarse step)
+  for (int l = c->mp.levelmin - 1; l >= 1; l--) RB_TRY(upload_fine_impl(c, l));
+  if (c->finest >= 1 && finest_alternates(c, c->finest)) RB_TRY(set_unew_impl(c, c->finest));  // unew = uold after a run
+  RB_CUDA(cudaEventRecord(c->ev1, c->stream));
   int64_t coarse = 0;
   RB_TRY(sched_download(c, &coarse));
   c->cell_updates += coarse * updates_per_coarse(c, c->mp.levelmin);
@@ -1621,7 +1724,7 @@ int rb_create(const rb_hydro_params* hp, const rb_mesh_params* mp, int precision
   if ((rc = dalloc(&c->d_uold, (size_t)c->ncell * 5)) || (rc = dalloc(&c->d_unew, (size_t)c->ncell * 5)) ||
       (rc = dalloc(&c->d_son, (size_t)c->ncell)) ||
       (rc = dalloc(&c->d_stage, (size_t)c->ncell * 5)) || (rc = dalloc(&c->d_red, 8)) ||
-      (rc = dalloc(&c->d_clock, 8)) || (rc = dalloc(&c->d_sched, RB_S_SIZE)))
+      (rc = dalloc(&c->d_clock, 8)) || (rc = dalloc(&c->d_sched, RB_S_SIZE)) || (rc = dalloc(&c->d_cfl, 2)))
     return bail(rc);
   if (c->hp.pressure_fix) {
     if ((rc = dalloc(&c->d_divu, (size_t)c->ncell)) || (rc = dalloc(&c->d_enew, (size_t)c->ncell))) return bail(rc);
@@ -1635,6 +1738,7 @@ int rb_create(const rb_hydro_params* hp, const rb_mesh_params* mp, int precision
   if (cudaMemsetAsync(c->d_uold, 0, (size_t)c->ncell * 5 * sizeof(double), c->stream) != cudaSuccess ||
       cudaMemsetAsync(c->d_unew, 0, (size_t)c->ncell * 5 * sizeof(double), c->stream) != cudaSuccess ||
       cudaMemsetAsync(c->d_clock, 0, 8 * sizeof(double), c->stream) != cudaSuccess ||
+      cudaMemsetAsync(c->d_cfl, 0, 2 * sizeof(unsigned long long), c->stream) != cudaSuccess ||
       cudaStreamSynchronize(c->stream) != cudaSuccess)
     return bail(fail(RB_ERR_CUDA, "initialising device buffers failed"));
   // make sure the kernel image for this GPU is present
@@ -1653,7 +1757,7 @@ int rb_destroy(rb_context* c) {
   c->table_pool = nullptr;
   dfree(c->d_uold); dfree(c->d_unew); dfree(c->d_son);
   dfree(c->d_divu); dfree(c->d_enew); dfree(c->d_bbuf);
-  dfree(c->d_stage); dfree(c->d_partial); dfree(c->d_red); dfree(c->d_clock); dfree(c->d_sched);
+  dfree(c->d_stage); dfree(c->d_partial); dfree(c->d_red); dfree(c->d_clock); dfree(c->d_sched); dfree(c->d_cfl);
   dfree(c->d_flag);
   if (c->h_red) cudaFreeHost(c->h_red);
   if (c->h_sched) cudaFreeHost(c->h_sched);
@@ -1961,13 +2065,11 @@ int rb_run(rb_context* c, int max_steps, double t_end, int use_graph, double* t_
     rb_context* c;
     ~GateScope() { c->gate = nullptr; }
   } scope{c};
+  RB_CUDA(cudaEventRecord(c->ev0, c->stream));
   RB_TRY(run_async_begin(c, t_end, max_steps));
   const int chunk = std::max(1, std::min(max_steps, 8));
-  RB_CUDA(cudaEventRecord(c->ev0, c->stream));
-  RB_CUDA(cudaEventRecord(c->ev1, c->stream));
   for (int64_t launched = 0; launched < max_steps;) {
     RB_TRY(run_async_chunk(c, chunk, use_graph != 0));
-    RB_CUDA(cudaEventRecord(c->ev1, c->stream));
     launched += chunk;
     RB_CUDA(cudaMemcpyAsync(c->h_sched, c->d_sched, RB_S_SIZE * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     RB_CUDA(cudaStreamSynchronize(c->stream));
@@ -1976,7 +2078,7 @@ int rb_run(rb_context* c, int max_steps, double t_end, int use_graph, double* t_
   }
   int64_t coarse = 0;
   RB_TRY(run_async_end(c, &coarse));
-  RB_CUDA(cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1));  // device time of all chunks
+  RB_CUDA(cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1));  // device time of the run
   if (t_io) *t_io = c->t;
   if (steps_done) *steps_done = (int)coarse;
   return RB_OK;

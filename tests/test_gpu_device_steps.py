@@ -1,0 +1,42 @@
+"""GPU: the device-scheduled coarse steps (rb_run) with subcycling patterns
+that do and do not let the finest level alternate its two buffers, against the
+host-scheduled coarse steps and the oracle, FP64 bit for bit."""
+import numpy as np
+import pytest
+
+import oracle
+from ramses_b200 import runtime
+
+from helpers import sedov_amr
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("levels", [(3, 3), (3, 4), (3, 6)])
+@pytest.mark.parametrize("pattern", [(2, 2), (1, 1), (1, 2), (2, 1)])
+def test_subcycling_patterns(cuda_lib, oracle_lib, levels, pattern):
+    """pattern: nsubcycle of the even and the odd levels; runs in chunks of
+    one, three and a stop in the middle of a graph of eight."""
+    tree, hp, u = sedov_amr(*levels)
+    ns = [pattern[i % 2] for i in range(33)]
+    orc = oracle.OracleRun(tree, hp, u, nsubcycle=ns)
+    with runtime.Solver(tree, hp, nsubcycle=ns, uold=u) as s:
+        for n in (1, 3):
+            assert s.run(max_steps=n) == n
+            for _ in range(n):
+                orc.coarse_step()
+            np.testing.assert_array_equal(s.download_state(), orc.uold)
+            assert s.t == orc.t
+        t_end = s.t * 1.5
+        steps = s.run(t_end=t_end, max_steps=50)
+        while orc.t < t_end:
+            orc.coarse_step()
+            steps -= 1
+        assert steps == 0
+        np.testing.assert_array_equal(s.download_state(), orc.uold)
+        assert s.t == orc.t
+        # the finest level's unew holds the state, as after set_uold
+        lf = max(l for l in range(1, tree.nlevelmax + 1) if tree.noct(l))
+        g = tree.active[lf].astype(np.int64)
+        cells = (tree.ncoarse + np.arange(8)[:, None] * tree.ngridmax + g[None, :] - 1).ravel()
+        np.testing.assert_array_equal(s.download_unew()[:, cells], orc.uold[:, cells])
