@@ -2,25 +2,33 @@
 // godfine1 :486-911 and unsplit, umuscl.f90:22-171) as a tiled sm_100a stencil.
 //
 // A tile is an aligned box of TX x TY x TZ level-l cells (TX/2 x TY/2 x TZ/2
-// octs). One CTA owns one tile:
+// octs). One CTA owns one tile, one thread one cell of it:
 //   A. gather the (TX+4)(TY+4)(TZ+4) stencil into shared memory as primitive
 //      variables. Each 2x2x2 block of the stencil is an existing level-l oct
 //      (read from uold), a prolongated coarse cell (interpol_hydro, computed
 //      beforehand into the interpolation buffer), or absent (no active oct
 //      reads it); plus the refinement flag son(cell)>0 of every cell;
-//   B. slopes + MUSCL-Hancock trace once per cell of the tile and of the
-//      one-cell face slabs around it;
+//   B. slopes + MUSCL-Hancock trace: every thread its own cell, whose states at
+//      the lower faces stay in registers and at the upper faces go to shared
+//      memory, then one cell of the one-cell face slabs around the tile;
 //   C. one Riemann problem per face, flux*dt/dx, zeroed where either side is
-//      refined (godunov_fine.f90:720-747);
+//      refined (godunov_fine.f90:720-747): every thread the three lower faces
+//      of its cell, then the upper faces of the tile's far sides;
 //   D. unew += (Fx_l - Fx_r) then y then z for the cells of active octs
-//      (godunov_fine.f90:751-792);
+//      (godunov_fine.f90:751-792), the lower fluxes from registers;
 //   E. the boundary-face fluxes of octs that border an unrefined coarser cell
 //      are stored for the deterministic fine-to-coarse correction.
 // Every quantity is a pure function of its stencil, so computing each cell
 // and face once per tile gives the values the reference computes (redundantly)
 // per oct.
+//
+// What bounds it: instruction issue (FP32-mixed) and the latency of the FP64
+// chains (drop-in), so what counts is instructions per cell and CTAs in
+// flight. States are packed for 128-bit shared accesses, and only one of a
+// face's two states passes through shared memory.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 #include "cp_async.cuh"
 #include "hydro_core.cuh"
@@ -60,7 +68,9 @@ struct TileArgs {
 // block code: >= 0 oct index (igrid-1); -1 absent; <= -2 interpolation entry (-code-2)
 template <int TX, int TY, int TZ>
 struct TileGeom {
-  static constexpr int SX = TX + 4, SY = TY + 4, SZ = TZ + 4;
+  // stencil; the row stride is odd, so that the x slabs' column accesses (16
+  // bytes per lane) fall into different banks
+  static constexpr int SX = TX + 5, SY = TY + 4, SZ = TZ + 4;
   static constexpr int NS = SX * SY * SZ;
   static constexpr int BX = TX / 2 + 2, BY = TY / 2 + 2, BZ = TZ / 2 + 2;
   static constexpr int NBLK = BX * BY * BZ;
@@ -70,8 +80,11 @@ struct TileGeom {
   static constexpr int NFZ = TX * TY * (TZ + 1);
   static constexpr int NF = NFX + NFY + NFZ;
   static constexpr int NCELL = TX * TY * TZ;
-  static constexpr int NTRACE = NCELL + 2 * (TY * TZ + TX * TZ + TX * TY);
-  static_assert(5 * NF <= 5 * NS, "flux must fit in the stencil buffer");
+  // one-cell face slabs: lower and upper side of x, y, z; the upper sides'
+  // faces are the tile's far faces
+  static constexpr int NUX = TY * TZ, NUY = TX * TZ, NUZ = TX * TY;
+  static constexpr int NU = NUX + NUY + NUZ;
+  static constexpr int NSLAB = 2 * NU;
 };
 
 // Stencil cells read by the slopes of types 0, 1, 2, 7 and 8: the tile, its
@@ -101,45 +114,197 @@ constexpr int gather_count() {
     for (int ch = 0; ch < 8; ch++) n += gather_children<TX, TY, TZ>(b, ch);
   return n;
 }
+// entry: stencil slot | block << 12 | child << 21 | (cell of the tile) << 24
+template <int TX, int TY, int TZ>
+constexpr uint32_t gather_entry(int b, int ch) {
+  using G = TileGeom<TX, TY, TZ>;
+  const int sx = 2 * (b % G::BX) + (ch & 1), sy = 2 * ((b / G::BX) % G::BY) + ((ch >> 1) & 1),
+            sz = 2 * (b / (G::BX * G::BY)) + (ch >> 2);
+  const bool inner = sx >= 2 && sx < 2 + TX && sy >= 2 && sy < 2 + TY && sz >= 2 && sz < 2 + TZ;
+  return (uint32_t)(sx + G::SX * (sy + G::SY * sz)) | (uint32_t)b << 12 | (uint32_t)ch << 21 | (uint32_t)inner << 24;
+}
 template <int TX, int TY, int TZ>
 struct GatherList {
   static constexpr int N = gather_count<TX, TY, TZ>();
-  uint16_t e[N];
+  static_assert(TileGeom<TX, TY, TZ>::NS <= 4096 && TileGeom<TX, TY, TZ>::NBLK <= 512, "entry fields");
+  uint32_t e[N];
   constexpr GatherList() : e{} {
     int n = 0;
     for (int b = 0; b < TileGeom<TX, TY, TZ>::NBLK; b++)
       for (int ch = 0; ch < 8; ch++)
-        if (gather_children<TX, TY, TZ>(b, ch)) e[n++] = (uint16_t)(b << 3 | ch);
+        if (gather_children<TX, TY, TZ>(b, ch)) e[n++] = gather_entry<TX, TY, TZ>(b, ch);
   }
 };
 template <int TX, int TY, int TZ>
 __device__ const GatherList<TX, TY, TZ> kGatherList{};
 
+// N five-value states in shared memory, packed for 128-bit accesses: float as
+// (r,u,v,w) + p, double as (r,u) + (v,w) + p.
+template <typename R> struct States;
+template <> struct States<float> {
+  float4* a;
+  float* b;
+  static constexpr __host__ __device__ int pad(int n) { return (n + 3) & ~3; }
+  static constexpr __host__ __device__ size_t bytes(int n) { return 20 * (size_t)pad(n); }
+  __device__ States(unsigned char* base, int n)
+      : a(reinterpret_cast<float4*>(base)), b(reinterpret_cast<float*>(base + 16 * (size_t)pad(n))) {}
+  __device__ __forceinline__ Prim<float> get(int i) const {
+    const float4 x = a[i];
+    return Prim<float>{x.x, x.y, x.z, x.w, b[i]};
+  }
+  __device__ __forceinline__ void put(int i, const Prim<float>& q) {
+    a[i] = make_float4(q.r, q.u, q.v, q.w);
+    b[i] = q.p;
+  }
+  __device__ __forceinline__ float& at(int i, int v) {
+    return v < 4 ? reinterpret_cast<float*>(a)[4 * i + v] : b[i];
+  }
+};
+template <> struct States<double> {
+  double2 *a, *b;
+  double* c;
+  static constexpr __host__ __device__ int pad(int n) { return (n + 1) & ~1; }
+  static constexpr __host__ __device__ size_t bytes(int n) { return 40 * (size_t)pad(n); }
+  __device__ States(unsigned char* base, int n)
+      : a(reinterpret_cast<double2*>(base)), b(reinterpret_cast<double2*>(base + 16 * (size_t)pad(n))),
+        c(reinterpret_cast<double*>(base + 32 * (size_t)pad(n))) {}
+  __device__ __forceinline__ Prim<double> get(int i) const {
+    const double2 x = a[i], y = b[i];
+    return Prim<double>{x.x, x.y, y.x, y.y, c[i]};
+  }
+  __device__ __forceinline__ void put(int i, const Prim<double>& q) {
+    a[i] = make_double2(q.r, q.u);
+    b[i] = make_double2(q.v, q.w);
+    c[i] = q.p;
+  }
+  __device__ __forceinline__ double& at(int i, int v) {
+    return v < 2 ? reinterpret_cast<double*>(a)[2 * i + v] : v < 4 ? reinterpret_cast<double*>(b)[2 * i + v - 2] : c[i];
+  }
+};
+
+// dynamic shared memory: the stencil's primitive states, reused for the face
+// fluxes once they are traced; the lower cell's state at every face; the
+// upper slab's state at the far faces; block codes; flags
+template <typename R, int TX, int TY, int TZ>
+struct TileSmem {
+  using G = TileGeom<TX, TY, TZ>;
+  static constexpr size_t Q = 0;
+  static constexpr size_t L = (States<R>::bytes(G::NS > G::NF ? G::NS : G::NF) + 15) & ~(size_t)15;
+  static constexpr size_t U = L + ((States<R>::bytes(G::NF) + 15) & ~(size_t)15);
+  static constexpr size_t BLK = U + ((States<R>::bytes(G::NU) + 15) & ~(size_t)15);
+  static constexpr size_t OK = BLK + sizeof(int32_t) * (size_t)G::NBLK;
+  static constexpr size_t SIZE = OK + (size_t)((G::NS + 15) & ~15);
+};
 template <typename R, int TX, int TY, int TZ>
 constexpr size_t tile_smem_bytes() {
+  return TileSmem<R, TX, TY, TZ>::SIZE;
+}
+
+// Traced face states of one cell from its state q0 and its neighbours in q
+// (stencil slot s): sp[d] at the lower, sm[d] at the upper face of direction d,
+// for the directions of mask.
+template <typename R, int TX, int TY, int TZ, int RS, int ST>
+__device__ __forceinline__ void trace_slot(const States<R>& q, int s, const Consts<R>& c, int slope_type,
+                                           const R dtd[3], unsigned mask, Prim<R> sp[3], Prim<R> sm[3]) {
   using G = TileGeom<TX, TY, TZ>;
-  // q/flux union + face states (M and P) + block codes + refinement flags
-  return sizeof(R) * (size_t)(5 * G::NS) + sizeof(R) * (size_t)(2 * 5 * G::NF) +
-         sizeof(int32_t) * (size_t)G::NBLK + (size_t)((G::NS + 15) & ~15);
+  constexpr int st[3] = {1, G::SX, G::SX * G::SY};
+  const Prim<R> q0 = q.get(s);
+  if constexpr (sizeof(R) == 4 && RS == RB_RIEMANN_HLLC && (ST == 1 || ST == 2)) {
+    float hd[5][3], h[5];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const Prim<float> a = q.get(s - st[d]), b = q.get(s + st[d]);
+      hd[0][d] = hslope<ST>(a.r, q0.r, b.r);
+      hd[1][d] = hslope<ST>(a.u, q0.u, b.u);
+      hd[2][d] = hslope<ST>(a.v, q0.v, b.v);
+      hd[3][d] = hslope<ST>(a.w, q0.w, b.w);
+      hd[4][d] = hslope<ST>(a.p, q0.p, b.p);
+    }
+    half_step(q0, hd, c.gamma, dtd[0], h);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      if (!(mask & (1u << d))) continue;
+      float P[5], M[5];
+      face_pair(h, hd, d, q0.r, c.smallr, P, M);
+      sp[d] = Prim<float>{P[0], P[1], P[2], P[3], P[4]};
+      sm[d] = Prim<float>{M[0], M[1], M[2], M[3], M[4]};
+    }
+  } else {
+    R dq[5][3];
+    if (slope_type == 0) {
+#pragma unroll
+      for (int v = 0; v < 5; v++) { dq[v][0] = (R)0; dq[v][1] = (R)0; dq[v][2] = (R)0; }
+    } else if (slope_type != 3) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        const Prim<R> a = q.get(s - st[d]), b = q.get(s + st[d]);
+        dq[0][d] = slope1<R>(a.r, q0.r, b.r, slope_type, c.slope_theta);
+        dq[1][d] = slope1<R>(a.u, q0.u, b.u, slope_type, c.slope_theta);
+        dq[2][d] = slope1<R>(a.v, q0.v, b.v, slope_type, c.slope_theta);
+        dq[3][d] = slope1<R>(a.w, q0.w, b.w, slope_type, c.slope_theta);
+        dq[4][d] = slope1<R>(a.p, q0.p, b.p, slope_type, c.slope_theta);
+      }
+    } else {
+      // positivity-preserving multidimensional slope (umuscl.f90:1328-1392)
+      const R half = (R)0.5, one = (R)1, zero = (R)0;
+      const R qc[5] = {q0.r, q0.u, q0.v, q0.w, q0.p};
+      R vmin[5], vmax[5];
+      bool first = true;
+      for (int kk = -1; kk <= 1; kk++)
+        for (int ii = -1; ii <= 1; ii++)
+          for (int jj = -1; jj <= 1; jj++) {
+            const Prim<R> n = q.get(s + ii + G::SX * (jj + G::SY * kk));
+            const R d[5] = {n.r - qc[0], n.u - qc[1], n.v - qc[2], n.w - qc[3], n.p - qc[4]};
+#pragma unroll
+            for (int v = 0; v < 5; v++) {
+              vmin[v] = first ? d[v] : fmn(vmin[v], d[v]);
+              vmax[v] = first ? d[v] : fmx(vmax[v], d[v]);
+            }
+            first = false;
+          }
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        const Prim<R> a = q.get(s - st[d]), b = q.get(s + st[d]);
+        dq[0][d] = half * (b.r - a.r);
+        dq[1][d] = half * (b.u - a.u);
+        dq[2][d] = half * (b.v - a.v);
+        dq[3][d] = half * (b.w - a.w);
+        dq[4][d] = half * (b.p - a.p);
+      }
+#pragma unroll
+      for (int v = 0; v < 5; v++) {
+        const R dff = half * ((R)fabs(dq[v][0]) + (R)fabs(dq[v][1]) + (R)fabs(dq[v][2]));
+        R slop;
+        if (dff > zero) slop = fmn(one, fmn((R)fabs(vmin[v]), (R)fabs(vmax[v])) / dff);
+        else slop = one;
+        dq[v][0] = slop * dq[v][0]; dq[v][1] = slop * dq[v][1]; dq[v][2] = slop * dq[v][2];
+      }
+    }
+    trace_sel<R, RS, ST>(q0, dq, c, dtd, sp, sm, mask);
+  }
 }
 
 // RS (Riemann solver) and ST (slope type) fix the scheme at compile time;
 // RS = 0 / ST = -1 read it from a.hp at run time. PF: pressure_fix, the
 // velocity-divergence and internal-energy fluxes of every face (umuscl.f90
 // cmpflxm's tmp, :845-849) update a.divu and a.enew beside unew
-// (godunov_fine.f90:735-744, 775-789).
-template <typename R, int TX, int TY, int TZ, int NT, int RS, int ST, bool PF = false>
-__global__ void __launch_bounds__(NT) godunov_tile_kernel(TileArgs a) {
+// (godunov_fine.f90:735-744, 775-789). MINB: CTAs per SM the registers are
+// bounded for.
+template <typename R, int TX, int TY, int TZ, int NT, int MINB, int RS, int ST, bool PF = false>
+__global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_constant__ TileArgs a) {
   using G = TileGeom<TX, TY, TZ>;
-  constexpr int SX = G::SX, SY = G::SY, NS = G::NS;
-  constexpr int BX = G::BX, BY = G::BY, NBLK = G::NBLK;
+  using M = TileSmem<R, TX, TY, TZ>;
+  constexpr int SX = G::SX, SY = G::SY;
+  constexpr int BX = G::BX, BY = G::BY, NBLK = G::NBLK, NCELL = G::NCELL;
   constexpr int NFX = G::NFX, NFY = G::NFY, NF = G::NF;
+  static_assert(NCELL <= NT, "one thread per cell");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  R* q = reinterpret_cast<R*>(smem_raw);                 // [5][NS]; reused as flux [5][NF]
-  R* qm = q + 5 * NS;                                    // [5][NF]
-  R* qp = qm + 5 * NF;                                   // [5][NF]
-  int32_t* blk = reinterpret_cast<int32_t*>(qp + 5 * NF);// [NBLK]
-  unsigned char* okf = reinterpret_cast<unsigned char*>(blk + NBLK);  // [NS]
+  States<R> q(smem_raw + M::Q, G::NS);       // stencil
+  States<R> F(smem_raw + M::Q, NF);          // fluxes, once the stencil is traced
+  States<R> Ls(smem_raw + M::L, NF);         // lower cell's state at a face
+  States<R> Us(smem_raw + M::U, G::NU);      // upper slab's state at a far face
+  int32_t* blk = reinterpret_cast<int32_t*>(smem_raw + M::BLK);
+  unsigned char* okf = smem_raw + M::OK;
 
   const int tile = blockIdx.x;
   if (tile >= a.ntile) return;
@@ -168,18 +333,16 @@ __global__ void __launch_bounds__(NT) godunov_tile_kernel(TileArgs a) {
 
   // ---- A. gather + ctoprim ------------------------------------------------
   const int slope_type = ST >= 0 ? ST % 10 : a.hp.slope_type;
-  const bool slope27 = (slope_type == 3);
   // the 27-point slopes and the corner divergence of difmag read the edge and
   // corner cells of the stencil too
-  const bool full_gather = slope27 || (RS == 0 && a.hp.difmag > 0.0);
+  const bool full_gather = slope_type == 3 || (RS == 0 && a.hp.difmag > 0.0);
   // one stencil cell: its raw state is loaded by gather_cell and converted by
   // put_cell (the listed gather keeps the loads of two cells in flight
   // before their conversion). Blocks coded -1 are read by no present cell:
   // only their flags are set.
-  auto gather_cell = [&](int b, int ch, double u[5], int& code, int& sonv, int& inner) -> int {
-    const int bx = b % BX, by = (b / BX) % BY, bz = b / (BX * BY);
-    const int sx = 2 * bx + (ch & 1), sy = 2 * by + ((ch >> 1) & 1), sz = 2 * bz + (ch >> 2);
-    code = blk[b];
+  auto gather_cell = [&](uint32_t e, double u[5], int& code, int& sonv) {
+    code = blk[(e >> 12) & 511];
+    const int ch = (e >> 21) & 7;
     sonv = 0;
     // L2-only loads: the tile reads each stencil cell once, and leaving L1
     // to the loads in flight lets more of them be outstanding
@@ -189,25 +352,17 @@ __global__ void __launch_bounds__(NT) godunov_tile_kernel(TileArgs a) {
       for (int v = 0; v < 5; v++) u[v] = __ldcg(a.uold + v * ncell + dc);
       if (a.has_refined) sonv = __ldcg(a.son + dc);
     } else if (code <= -2) {
-      const int64_t e = (int64_t)(-code - 2) * 8 + ch;
+      const int64_t i = (int64_t)(-code - 2) * 8 + ch;
 #pragma unroll
-      for (int v = 0; v < 5; v++) u[v] = __ldcg(a.interp + v * a.ninterp8 + e);
+      for (int v = 0; v < 5; v++) u[v] = __ldcg(a.interp + v * a.ninterp8 + i);
     }
-    // a tile-interior cell of a present oct (its faces and update are used)
-    inner = sx >= 2 && sx < 2 + TX && sy >= 2 && sy < 2 + TY && sz >= 2 && sz < 2 + TZ && code >= 0;
-    return sx + SX * (sy + SY * sz);
   };
-  auto put_cell = [&](int s, const double u[5], int code, int sonv, int inner) {
+  auto put_cell = [&](uint32_t e, const double u[5], int code, int sonv) {
+    const int s = e & 4095;
     // okf bit 0: the cell is refined (its faces carry no flux); bit 1: a
-    // tile-interior cell of a present oct
-    okf[s] = (unsigned char)((sonv > 0 ? 1 : 0) | (inner ? 2 : 0));
-    if (code == -1) return;
-    const Prim<R> pq = ctoprim_cell<R>(u, a.hp);
-    q[0 * NS + s] = pq.r;
-    q[1 * NS + s] = pq.u;
-    q[2 * NS + s] = pq.v;
-    q[3 * NS + s] = pq.w;
-    q[4 * NS + s] = pq.p;
+    // tile-interior cell of a present oct (its faces and update are used)
+    okf[s] = (unsigned char)((sonv > 0 ? 1 : 0) | ((e >> 24) && code >= 0 ? 2 : 0));
+    if (code != -1) q.put(s, ctoprim_cell<R>(u, a.hp));
   };
   if (!full_gather) {
     using GL = GatherList<TX, TY, TZ>;
@@ -216,129 +371,89 @@ __global__ void __launch_bounds__(NT) godunov_tile_kernel(TileArgs a) {
     constexpr int NB = PER < 2 ? PER : 2;
     for (int j0 = 0; j0 < PER; j0 += NB) {
       double u[NB][5];
-      int sidx[NB], code[NB], sonv[NB], inner[NB];
+      uint32_t e[NB];
+      int code[NB], sonv[NB];
 #pragma unroll
       for (int j = 0; j < NB; j++) {
         const int it = tid + (j0 + j) * NT;
-        sidx[j] = -1;
+        e[j] = ~0u;
         if (j0 + j < PER && it < NG) {
-          const int e = __ldg(&kGatherList<TX, TY, TZ>.e[it]);
-          sidx[j] = gather_cell(e >> 3, e & 7, u[j], code[j], sonv[j], inner[j]);
+          e[j] = __ldg(&kGatherList<TX, TY, TZ>.e[it]);
+          gather_cell(e[j], u[j], code[j], sonv[j]);
         }
       }
 #pragma unroll
       for (int j = 0; j < NB; j++)
-        if (sidx[j] >= 0) put_cell(sidx[j], u[j], code[j], sonv[j], inner[j]);
+        if (e[j] != ~0u) put_cell(e[j], u[j], code[j], sonv[j]);
     }
   } else {
     // every cell of the stencil
     for (int it = tid; it < NBLK * 8; it += NT) {
+      const int b = it >> 3, ch = it & 7;
+      const int sx = 2 * (b % BX) + (ch & 1), sy = 2 * ((b / BX) % BY) + ((ch >> 1) & 1), sz = 2 * (b / (BX * BY)) + (ch >> 2);
+      const bool inner = sx >= 2 && sx < 2 + TX && sy >= 2 && sy < 2 + TY && sz >= 2 && sz < 2 + TZ;
+      const uint32_t e = (uint32_t)(sx + SX * (sy + SY * sz)) | (uint32_t)b << 12 | (uint32_t)ch << 21 | (uint32_t)inner << 24;
       double u[5];
-      int code, sonv, inner;
-      const int s = gather_cell(it >> 3, it & 7, u, code, sonv, inner);
-      put_cell(s, u, code, sonv, inner);
+      int code, sonv;
+      gather_cell(e, u, code, sonv);
+      put_cell(e, u, code, sonv);
     }
   }
   __syncthreads();
 
   // ---- B. slopes + trace ----------------------------------------------------
   const double dt = a.dt_dev ? *a.dt_dev : a.dt;
-  R dtd[3];
-  {
-    const double dtdx = dt / a.dx;  // trace3d.f90 dtdx = dt/dx (dx=dy=dz)
-    dtd[0] = dtd[1] = dtd[2] = (R)dtdx;
+  const R dtdx = (R)(dt / a.dx);  // trace3d.f90 dtdx = dt/dx (dx=dy=dz)
+  const R dtd[3] = {dtdx, dtdx, dtdx};
+  // this thread's cell; x fastest, so that a quarter warp's 16-byte shared
+  // accesses are consecutive and a warp's global rows whole 32-byte sectors
+  const bool own = tid < NCELL;
+  const int x = tid % TX, y = (tid / TX) % TY, z = (tid / (TX * TY)) % TZ;
+  const int s_own = (x + 2) + SX * ((y + 2) + SY * (z + 2));
+  const int code_own = own ? blk[(x / 2 + 1) + BX * ((y / 2 + 1) + BY * (z / 2 + 1))] : -1;
+  // lower faces of the own cell
+  const int fx0 = x + (TX + 1) * (y + TY * z);
+  const int fy0 = NFX + x + TX * (y + (TY + 1) * z);
+  const int fz0 = NFX + NFY + x + TX * (y + TY * z);
+  Prim<R> P[3];
+  if (code_own != -1) {
+    Prim<R> sm[3];
+    trace_slot<R, TX, TY, TZ, RS, ST>(q, s_own, c, slope_type, dtd, 7u, P, sm);
+    Ls.put(fx0 + 1, sm[0]);
+    Ls.put(fy0 + TX, sm[1]);
+    Ls.put(fz0 + TX * TY, sm[2]);
   }
-  // present(x,y,z): the tile-interior cell belongs to an oct of this level
+  // present(s): the tile-interior cell belongs to an oct of this level
   // (its update and its faces are used; bit 1 of okf). A block coded -1 is
   // absent and not a stencil source of any present oct, so no face touching
   // it is used.
-  auto present = [&](int x, int y, int z) { return (okf[(x + 2) + SX * ((y + 2) + SY * (z + 2))] & 2) != 0; };
-  for (int it = tid; it < G::NTRACE; it += NT) {
-    int x, y, z;
-    unsigned mask;
-    if (it < G::NCELL) {
-      x = it % TX; y = (it / TX) % TY; z = it / (TX * TY); mask = 7u;
-      if (blk[(x / 2 + 1) + BX * ((y / 2 + 1) + BY * (z / 2 + 1))] == -1) continue;
+#pragma unroll 1
+  for (int it = tid; it < G::NSLAB; it += NT) {
+    const int side = it >= G::NU, r = side ? it - G::NU : it;
+    int s, d, f;  // slab slot, direction, face towards the tile
+    if (r < G::NUX) {
+      const int yy = r % TY, zz = r / TY;
+      d = 0; s = (side ? TX + 2 : 1) + SX * ((yy + 2) + SY * (zz + 2)); f = (TX + 1) * (yy + TY * zz);
+    } else if (r < G::NUX + G::NUY) {
+      const int k = r - G::NUX, xx = k % TX, zz = k / TX;
+      d = 1; s = (xx + 2) + SX * ((side ? TY + 2 : 1) + SY * (zz + 2)); f = NFX + xx + TX * (TY + 1) * zz;
     } else {
-      int r = it - G::NCELL;
-      if (r < 2 * TY * TZ) {           // x slabs: x = -1 (qm only) and x = TX (qp only)
-        const int side = r / (TY * TZ); r %= TY * TZ;
-        x = side ? TX : -1; y = r % TY; z = r / TY; mask = 1u;
-        if (!present(side ? TX - 1 : 0, y, z)) continue;
-      } else if ((r -= 2 * TY * TZ) < 2 * TX * TZ) {
-        const int side = r / (TX * TZ); r %= TX * TZ;
-        y = side ? TY : -1; x = r % TX; z = r / TX; mask = 2u;
-        if (!present(x, side ? TY - 1 : 0, z)) continue;
-      } else {
-        r -= 2 * TX * TZ;
-        const int side = r / (TX * TY); r %= TX * TY;
-        z = side ? TZ : -1; x = r % TX; y = r / TX; mask = 4u;
-        if (!present(x, y, side ? TZ - 1 : 0)) continue;
-      }
+      const int k = r - G::NUX - G::NUY, xx = k % TX, yy = k / TX;
+      d = 2; s = (xx + 2) + SX * ((yy + 2) + SY * (side ? TZ + 2 : 1)); f = NFX + NFY + xx + TX * yy;
     }
-    const int s = (x + 2) + SX * ((y + 2) + SY * (z + 2));
-    R dq[5][3];
-    Prim<R> q0;
-    q0.r = q[s]; q0.u = q[NS + s]; q0.v = q[2 * NS + s]; q0.w = q[3 * NS + s]; q0.p = q[4 * NS + s];
-    if (slope_type == 0) {
-#pragma unroll
-      for (int v = 0; v < 5; v++) { dq[v][0] = (R)0; dq[v][1] = (R)0; dq[v][2] = (R)0; }
-    } else if (!slope27) {
-      constexpr int st[3] = {1, SX, SX * SY};
-#pragma unroll
-      for (int v = 0; v < 5; v++) {
-        const R* qv = q + v * NS;
-        const R qc = qv[s];
-#pragma unroll
-        for (int d = 0; d < 3; d++)
-          dq[v][d] = slope1<R>(qv[s - st[d]], qc, qv[s + st[d]], slope_type, c.slope_theta);
-      }
-    } else {
-      // positivity-preserving multidimensional slope (umuscl.f90:1328-1392)
-      const R half = (R)0.5, one = (R)1, zero = (R)0;
-#pragma unroll
-      for (int v = 0; v < 5; v++) {
-        const R* qv = q + v * NS;
-        const R qc = qv[s];
-        R vmin = (R)0, vmax = (R)0;
-        bool first = true;
-        for (int kk = -1; kk <= 1; kk++)
-          for (int ii = -1; ii <= 1; ii++)
-            for (int jj = -1; jj <= 1; jj++) {
-              const R d = qv[s + ii + SX * (jj + SY * kk)] - qc;
-              if (first) { vmin = d; vmax = d; first = false; }
-              else { vmin = fmn(vmin, d); vmax = fmx(vmax, d); }
-            }
-        const R dfx = half * (qv[s + 1] - qv[s - 1]);
-        const R dfy = half * (qv[s + SX] - qv[s - SX]);
-        const R dfz = half * (qv[s + SX * SY] - qv[s - SX * SY]);
-        const R dff = half * ((R)fabs(dfx) + (R)fabs(dfy) + (R)fabs(dfz));
-        R slop;
-        if (dff > zero) slop = fmn(one, fmn((R)fabs(vmin), (R)fabs(vmax)) / dff);
-        else slop = one;
-        dq[v][0] = slop * dfx; dq[v][1] = slop * dfy; dq[v][2] = slop * dfz;
-      }
-    }
+    const int step = d == 0 ? 1 : d == 1 ? SX : SX * SY;
+    if (!(okf[side ? s - step : s + step] & 2)) continue;
     Prim<R> sp[3], sm[3];
-    trace_sel<R, RS, ST>(q0, dq, c, dtd, sp, sm, mask);
-    // store: qm of direction d at face index (coord+1), qp at face index coord
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      if (!(mask & (1u << d))) continue;
-      int off, fm, fp;
-      if (d == 0) { off = 0;         fm = (x + 1) + (TX + 1) * (y + TY * z); fp = x + (TX + 1) * (y + TY * z); }
-      else if (d == 1) { off = NFX;  fm = x + TX * ((y + 1) + (TY + 1) * z); fp = x + TX * (y + (TY + 1) * z); }
-      else { off = NFX + NFY;        fm = x + TX * (y + TY * (z + 1));       fp = x + TX * (y + TY * z); }
-      const bool wm = (d == 0) ? (x < TX) : (d == 1) ? (y < TY) : (z < TZ);
-      const bool wp = (d == 0) ? (x >= 0) : (d == 1) ? (y >= 0) : (z >= 0);
-      if (wm) {
-        qm[0 * NF + off + fm] = sm[d].r; qm[1 * NF + off + fm] = sm[d].u; qm[2 * NF + off + fm] = sm[d].v;
-        qm[3 * NF + off + fm] = sm[d].w; qm[4 * NF + off + fm] = sm[d].p;
-      }
-      if (wp) {
-        qp[0 * NF + off + fp] = sp[d].r; qp[1 * NF + off + fp] = sp[d].u; qp[2 * NF + off + fp] = sp[d].v;
-        qp[3 * NF + off + fp] = sp[d].w; qp[4 * NF + off + fp] = sp[d].p;
-      }
+    trace_slot<R, TX, TY, TZ, RS, ST>(q, s, c, slope_type, dtd, 1u << d, sp, sm);
+    // lower slab: the left state of its face; upper slab: the right state
+    if (side) {
+      if (d == 0) Us.put(r, sp[0]);
+      else if (d == 1) Us.put(r, sp[1]);
+      else Us.put(r, sp[2]);
+    } else {
+      if (d == 0) Ls.put(f, sm[0]);
+      else if (d == 1) Ls.put(f, sm[1]);
+      else Ls.put(f, sm[2]);
     }
   }
   // difmag > 0 (run-time scheme variant): cmpdivu (uplmde.f90:702-764), the
@@ -353,9 +468,9 @@ __global__ void __launch_bounds__(NT) godunov_tile_kernel(TileArgs a) {
       const R quarter = (R)0.5 * (R)0.5;
       const R fxd = (R)(quarter / (R)a.dx), fyd = fxd, fzd = fxd;
       for (int it = tid; it < NCORN; it += NT) {
-        const int x = it % CXN, y = (it / CXN) % CYN, z = it / (CXN * CYN);
+        const int cx = it % CXN, cy = (it / CXN) % CYN, cz = it / (CXN * CYN);
         auto Q = [&](int ox, int oy, int oz, int v) {
-          return q[v * NS + (x + ox + 2) + SX * ((y + oy + 2) + SY * (z + oz + 2))];
+          return q.at((cx + ox + 2) + SX * ((cy + oy + 2) + SY * (cz + oz + 2)), v);
         };
         R ux = (R)0, vy = (R)0, wz = (R)0;
         ux = ux + fxd * (Q(0, 0, 0, 1) - Q(-1, 0, 0, 1));
@@ -372,9 +487,8 @@ __global__ void __launch_bounds__(NT) godunov_tile_kernel(TileArgs a) {
   __syncthreads();
 
   // ---- C. Riemann fluxes (flux buffer aliases q) ------------------------------
-  // raw (conservative) state of stencil cell s, as phase A gathered it
-  auto raw_cell = [&](int s, double u[5]) {
-    const int sx = s % SX, sy = (s / SX) % SY, sz = s / (SX * SY);
+  // raw (conservative) state of stencil cell (sx, sy, sz), as phase A gathered it
+  auto raw_cell = [&](int sx, int sy, int sz, double u[5]) {
     const int b = (sx >> 1) + BX * ((sy >> 1) + BY * (sz >> 1));
     const int ch = (sx & 1) + 2 * (sy & 1) + 4 * (sz & 1);
     const int code = blk[b];
@@ -388,75 +502,106 @@ __global__ void __launch_bounds__(NT) godunov_tile_kernel(TileArgs a) {
       for (int v = 0; v < 5; v++) u[v] = 0.0;
     }
   };
-  R* F = q;
-  for (int f = tid; f < NF; f += NT) {
-    int d, x, y, z;
-    if (f < NFX) { d = 0; x = f % (TX + 1); y = (f / (TX + 1)) % TY; z = f / ((TX + 1) * TY); }
-    else if (f < NFX + NFY) { const int r = f - NFX; d = 1; x = r % TX; y = (r / TX) % (TY + 1); z = r / (TX * (TY + 1)); }
-    else { const int r = f - NFX - NFY; d = 2; x = r % TX; y = (r / TX) % TY; z = r / (TX * TY); }
-    // the face between cell (x,y,z) and its lower neighbour along d is used
-    // only when one of the two is a present cell
-    const int sr = (x + 2) + SX * ((y + 2) + SY * (z + 2));
-    const int sl = sr - (d == 0 ? 1 : d == 1 ? SX : SX * SY);
-    const int fl = okf[sl] | okf[sr];
-    if (!(fl & 2)) continue;
-    Prim<R> L, Rr;
-    L.r = qm[f]; L.u = qm[NF + f]; L.v = qm[2 * NF + f]; L.w = qm[3 * NF + f]; L.p = qm[4 * NF + f];
-    Rr.r = qp[f]; Rr.u = qp[NF + f]; Rr.v = qp[2 * NF + f]; Rr.w = qp[3 * NF + f]; Rr.p = qp[4 * NF + f];
-    R ql[5], qr[5], fg[6], fo[5];
-    to_face(L, d, ql);
-    to_face(Rr, d, qr);
-    riemann_sel<R, RS>(ql, qr, c, fg);
-    from_face(fg, d, fo);
+  const float smallc2 = (float)c.smallc * (float)c.smallc;
+  auto scaled = [&](R v) -> R {
+    if (sizeof(R) == 8) {
+      // flux = fx*dt/dx, evaluated as (fx*dt)/dx (umuscl.f90:101-163);
+      // division by an exact power of two equals the multiplication
+      const double t = (double)v * dt;
+      return (R)(a.dx_pow2 ? t * a.inv_dx : t / a.dx);
+    }
+    return v * dtdx;
+  };
+  // The flux through face f between cell (cx, cy, cz) and its lower
+  // neighbour along D, from the states L and Rr: into F (and tmp, with
+  // pressure_fix, into Ls[f], which only this thread reads and has read).
+  auto face_flux = [&](auto dir, int f, int cx, int cy, int cz, const Prim<R>& L, const Prim<R>& Rr, int fl,
+                       Prim<R>& out, R tmp[2]) {
+    constexpr int D = decltype(dir)::value;
     // refined interface: either neighbour cell refined -> zero flux
     const bool zero_face = (fl & 1) != 0;
-    auto scaled = [&](R x) -> R {
-      if (sizeof(R) == 8) {
-        // flux = fx*dt/dx, evaluated as (fx*dt)/dx (umuscl.f90:101-163);
-        // division by an exact power of two equals the multiplication
-        const double t = (double)x * dt;
-        return (R)(a.dx_pow2 ? t * a.inv_dx : t / a.dx);
-      }
-      return x * dtd[0];
-    };
+    R ql[5], qr[5], fg[6], fo[5];
+    to_face(L, D, ql);
+    to_face(Rr, D, qr);
+    if constexpr (sizeof(R) == 4 && RS == RB_RIEMANN_HLLC && (ST == 1 || ST == 2)) {
+      hllc_f32<PF>(ql, qr, c, smallc2, dtdx, fg);
+      from_face(fg, D, fo);
+      if (PF) tmp[1] = zero_face ? (R)0 : fg[5];
+    } else {
+      riemann_sel<R, RS>(ql, qr, c, fg);
+      from_face(fg, D, fo);
+#pragma unroll
+      for (int v = 0; v < 5; v++) fo[v] = scaled(fo[v]);
+      if (PF) tmp[1] = zero_face ? (R)0 : scaled(fg[5]);
+    }
+    if (PF) tmp[0] = zero_face ? (R)0 : scaled((R)0.5 * (ql[1] + qr[1]));
     if (RS == 0 && a.hp.difmag > 0.0) {
       // consup (uplmde.f90:769-866): + dt*difmag*min(0, div1)*(u_R - u_L)
       // with div1 the mean of the face's four corner divergences, added
       // before the refined-face zeroing
       const R quarter = (R)0.5 * (R)0.5;
-      auto D = [&](int cx, int cy, int cz) { return cdiv[cx + CXN * (cy + CYN * cz)]; };
+      auto DV = [&](int ix, int iy, int iz) { return cdiv[ix + CXN * (iy + CYN * iz)]; };
       R div1;
-      if (d == 0) {
-        div1 = quarter * D(x, y, z);
-        div1 = div1 + quarter * D(x, y + 1, z);
-        div1 = div1 + quarter * (D(x, y, z + 1) + D(x, y + 1, z + 1));
-      } else if (d == 1) {
+      if (D == 0) {
+        div1 = quarter * DV(cx, cy, cz);
+        div1 = div1 + quarter * DV(cx, cy + 1, cz);
+        div1 = div1 + quarter * (DV(cx, cy, cz + 1) + DV(cx, cy + 1, cz + 1));
+      } else if (D == 1) {
         div1 = (R)0;
-        div1 = div1 + quarter * (D(x, y, z) + D(x + 1, y, z));
-        div1 = div1 + quarter * (D(x, y, z + 1) + D(x + 1, y, z + 1));
+        div1 = div1 + quarter * (DV(cx, cy, cz) + DV(cx + 1, cy, cz));
+        div1 = div1 + quarter * (DV(cx, cy, cz + 1) + DV(cx + 1, cy, cz + 1));
       } else {
-        div1 = quarter * (D(x, y, z) + D(x + 1, y, z) + D(x, y + 1, z) + D(x + 1, y + 1, z));
+        div1 = quarter * (DV(cx, cy, cz) + DV(cx + 1, cy, cz) + DV(cx, cy + 1, cz) + DV(cx + 1, cy + 1, cz));
       }
       div1 = (R)a.hp.difmag * fmn((R)0, div1);
       double ul[5], ur[5];
-      raw_cell(sl, ul);
-      raw_cell(sr, ur);
+      raw_cell(cx + 2 - (D == 0), cy + 2 - (D == 1), cz + 2 - (D == 2), ul);
+      raw_cell(cx + 2, cy + 2, cz + 2, ur);
 #pragma unroll
       for (int v = 0; v < 5; v++) {
         const R t = sizeof(R) == 8 ? (R)((double)(dt * (double)div1) * (ur[v] - ul[v]))
                                    : (R)(dt * (double)div1 * (ur[v] - ul[v]));
-        F[v * NF + f] = zero_face ? (R)0 : scaled(fo[v]) + t;
+        fo[v] = fo[v] + t;
       }
-    } else {
-#pragma unroll
-      for (int v = 0; v < 5; v++) F[v * NF + f] = zero_face ? (R)0 : scaled(fo[v]);
     }
+    if (zero_face) {
+#pragma unroll
+      for (int v = 0; v < 5; v++) fo[v] = (R)0;
+    }
+    out = Prim<R>{fo[0], fo[1], fo[2], fo[3], fo[4]};
+    F.put(f, out);
     if (PF) {
-      // tmp: the face-normal velocity average and the internal-energy flux,
-      // kept in this face's qm slots (read above, by this thread only)
-      const R half = (R)0.5;
-      qm[f] = zero_face ? (R)0 : scaled(half * (ql[1] + qr[1]));
-      qm[NF + f] = zero_face ? (R)0 : scaled(fg[5]);
+      Ls.at(f, 0) = tmp[0];
+      Ls.at(f, 1) = tmp[1];
+    }
+  };
+  // a face is used only when one of its two cells is a present cell
+  Prim<R> flo[3];    // fluxes through the own cell's lower faces
+  R tlo[3][2] = {{(R)0, (R)0}, {(R)0, (R)0}, {(R)0, (R)0}};
+  if (own) {
+    const int fo_ = okf[s_own];
+    const int fl0 = fo_ | okf[s_own - 1], fl1 = fo_ | okf[s_own - SX], fl2 = fo_ | okf[s_own - SX * SY];
+    if (fl0 & 2) face_flux(std::integral_constant<int, 0>(), fx0, x, y, z, Ls.get(fx0), P[0], fl0, flo[0], tlo[0]);
+    if (fl1 & 2) face_flux(std::integral_constant<int, 1>(), fy0, x, y, z, Ls.get(fy0), P[1], fl1, flo[1], tlo[1]);
+    if (fl2 & 2) face_flux(std::integral_constant<int, 2>(), fz0, x, y, z, Ls.get(fz0), P[2], fl2, flo[2], tlo[2]);
+  }
+  // the tile's far faces
+#pragma unroll 1
+  for (int r = tid; r < G::NU; r += NT) {
+    Prim<R> fo;
+    R t[2];
+    if (r < G::NUX) {
+      const int yy = r % TY, zz = r / TY, s = (TX + 2) + SX * ((yy + 2) + SY * (zz + 2));
+      const int f = TX + (TX + 1) * (yy + TY * zz), fl = okf[s - 1] | okf[s];
+      if (fl & 2) face_flux(std::integral_constant<int, 0>(), f, TX, yy, zz, Ls.get(f), Us.get(r), fl, fo, t);
+    } else if (r < G::NUX + G::NUY) {
+      const int k = r - G::NUX, xx = k % TX, zz = k / TX, s = (xx + 2) + SX * ((TY + 2) + SY * (zz + 2));
+      const int f = NFX + xx + TX * (TY + (TY + 1) * zz), fl = okf[s - SX] | okf[s];
+      if (fl & 2) face_flux(std::integral_constant<int, 1>(), f, xx, TY, zz, Ls.get(f), Us.get(r), fl, fo, t);
+    } else {
+      const int k = r - G::NUX - G::NUY, xx = k % TX, yy = k / TX, s = (xx + 2) + SX * ((yy + 2) + SY * (TZ + 2));
+      const int f = NFX + NFY + xx + TX * (yy + TY * TZ), fl = okf[s - SX * SY] | okf[s];
+      if (fl & 2) face_flux(std::integral_constant<int, 2>(), f, xx, yy, TZ, Ls.get(f), Us.get(r), fl, fo, t);
     }
   }
   cp_async_wait<0>();  // this thread's correction entries (E)
@@ -464,59 +609,55 @@ __global__ void __launch_bounds__(NT) godunov_tile_kernel(TileArgs a) {
 
   // ---- D. conservative update of active octs ----------------------------------
   double smax = 0.0, mass = 0.0, etot = 0.0, eint = 0.0;
-  const double vol = a.dx * a.dx * a.dx;
-  for (int it = tid; it < G::NCELL; it += NT) {
-    // octs-major order: 8 consecutive threads update one oct (coalesced rows)
-    const int o = it >> 3, ch = it & 7;
-    const int ox = o % (TX / 2), oy = (o / (TX / 2)) % (TY / 2), oz = o / ((TX / 2) * (TY / 2));
-    const int code = blk[(ox + 1) + BX * ((oy + 1) + BY * (oz + 1))];
-    if (code < 0) continue;
-    const int x = 2 * ox + (ch & 1), y = 2 * oy + ((ch >> 1) & 1), z = 2 * oz + (ch >> 2);
-    const int fxl = x + (TX + 1) * (y + TY * z);
-    const int fyl = NFX + x + TX * (y + (TY + 1) * z);
-    const int fzl = NFX + NFY + x + TX * (y + TY * z);
-    const int64_t dc = (int64_t)a.ncoarse + (int64_t)code * 8 + ch;
+  if (code_own >= 0) {
+    const int ch = (x & 1) + 2 * (y & 1) + 4 * (z & 1);
+    const int64_t dc = (int64_t)a.ncoarse + (int64_t)code_own * 8 + ch;
+    const Prim<R> fxr = F.get(fx0 + 1), fyr = F.get(fy0 + TX), fzr = F.get(fz0 + TX * TY);
+    const R fl[3][5] = {{flo[0].r, flo[0].u, flo[0].v, flo[0].w, flo[0].p},
+                        {flo[1].r, flo[1].u, flo[1].v, flo[1].w, flo[1].p},
+                        {flo[2].r, flo[2].u, flo[2].v, flo[2].w, flo[2].p}};
+    const R fr[3][5] = {{fxr.r, fxr.u, fxr.v, fxr.w, fxr.p},
+                        {fyr.r, fyr.u, fyr.v, fyr.w, fyr.p},
+                        {fzr.r, fzr.u, fzr.v, fzr.w, fzr.p}};
     double unv[5];
 #pragma unroll
-    for (int v = 0; v < 5; v++) {
-      const R* Fv = F + v * NF;
-      double un = a.fused ? __ldcg(a.uold + v * ncell + dc) : a.unew[v * ncell + dc];  // set_unew's value
-      un = un + ((double)Fv[fxl] - (double)Fv[fxl + 1]);
-      un = un + ((double)Fv[fyl] - (double)Fv[fyl + TX]);
-      un = un + ((double)Fv[fzl] - (double)Fv[fzl + TX * TY]);
-      a.unew[v * ncell + dc] = un;
-      unv[v] = un;
-    }
+    for (int v = 0; v < 5; v++) unv[v] = a.fused ? __ldcg(a.uold + v * ncell + dc) : a.unew[v * ncell + dc];  // set_unew's value
+    double dv = 0.0, en = 0.0;
     if (PF) {
       // divu, then enew, each x then y then z, as unew (the fused form
       // starts them from set_unew's values: 0 and the internal energy of uold)
-      const R* T1 = qm;
-      const R* T2 = qm + NF;
-      double dv, en;
       if (a.fused) {
-        double uo[5];
-#pragma unroll
-        for (int v = 0; v < 5; v++) uo[v] = __ldcg(a.uold + v * ncell + dc);
-        const double d = fmx(uo[0], a.hp.smallr);
-        const double uu = uo[1] / d, vv = uo[2] / d, ww = uo[3] / d;
-        dv = 0.0;
-        en = uo[4] - 0.5 * d * (uu * uu + vv * vv + ww * ww);
+        const double dd = fmx(unv[0], a.hp.smallr);
+        const double uu = unv[1] / dd, vv = unv[2] / dd, ww = unv[3] / dd;
+        en = unv[4] - 0.5 * dd * (uu * uu + vv * vv + ww * ww);
       } else {
         dv = a.divu[dc];
         en = a.enew[dc];
       }
-      dv = dv + ((double)T1[fxl] - (double)T1[fxl + 1]);
-      dv = dv + ((double)T1[fyl] - (double)T1[fyl + TX]);
-      dv = dv + ((double)T1[fzl] - (double)T1[fzl + TX * TY]);
-      en = en + ((double)T2[fxl] - (double)T2[fxl + 1]);
-      en = en + ((double)T2[fyl] - (double)T2[fyl + TX]);
-      en = en + ((double)T2[fzl] - (double)T2[fzl + TX * TY]);
+    }
+#pragma unroll
+    for (int v = 0; v < 5; v++) {
+      double un = unv[v];
+      un = un + ((double)fl[0][v] - (double)fr[0][v]);
+      un = un + ((double)fl[1][v] - (double)fr[1][v]);
+      un = un + ((double)fl[2][v] - (double)fr[2][v]);
+      a.unew[v * ncell + dc] = un;
+      unv[v] = un;
+    }
+    if (PF) {
+      dv = dv + ((double)tlo[0][0] - (double)Ls.at(fx0 + 1, 0));
+      dv = dv + ((double)tlo[1][0] - (double)Ls.at(fy0 + TX, 0));
+      dv = dv + ((double)tlo[2][0] - (double)Ls.at(fz0 + TX * TY, 0));
+      en = en + ((double)tlo[0][1] - (double)Ls.at(fx0 + 1, 1));
+      en = en + ((double)tlo[1][1] - (double)Ls.at(fy0 + TX, 1));
+      en = en + ((double)tlo[2][1] - (double)Ls.at(fz0 + TX * TY, 1));
       a.divu[dc] = dv;
       a.enew[dc] = en;
     }
     if (a.fused == 1) {
       // courant_fine on the updated state (the next step's CFL condition);
       // the level minimum of dt_cell is dt_cell(maximum wave speed)
+      const double vol = a.dx * a.dx * a.dx;
       const double ir = 1.0 / fmx(unv[0], a.hp.smallr);
       mass = mass + unv[0] * vol;
       etot = etot + unv[4] * vol;
@@ -559,8 +700,8 @@ __global__ void __launch_bounds__(NT) godunov_tile_kernel(TileArgs a) {
       if (d == 0) { const int fx = 2 * ox + 2 * side; fidx = fx + (TX + 1) * ((2 * oy + t1) + TY * (2 * oz + t2)); }
       else if (d == 1) { const int fy = 2 * oy + 2 * side; fidx = NFX + (2 * ox + t1) + TX * (fy + (TY + 1) * (2 * oz + t2)); }
       else { const int fz = 2 * oz + 2 * side; fidx = NFX + NFY + (2 * ox + t1) + TX * ((2 * oy + t2) + TY * fz); }
-      a.corr_flux[(int64_t)slot * 120 + face * 20 + r] = (double)F[v * NF + fidx];
-      if (PF && v < 2) a.corr_tmp[(int64_t)slot * 48 + face * 8 + cc * 2 + v] = (double)qm[v * NF + fidx];
+      a.corr_flux[(int64_t)slot * 120 + face * 20 + r] = (double)F.at(fidx, v);
+      if (PF && v < 2) a.corr_tmp[(int64_t)slot * 48 + face * 8 + cc * 2 + v] = (double)Ls.at(fidx, v);
     }
   }
 }

@@ -261,11 +261,18 @@ bool shape_fits(const rb_context* c, int l, int shape) {
   return true;
 }
 
+// Default tile shape of a level. 8x8x4 cells trace the fewest slab cells per
+// cell among the shapes that leave three (FP32-mixed) or two (FP64) CTAs per
+// SM: on 412 k octs 334 us against 344 (8x4x4), 402 (4x4x4) and 479 (8x8x8)
+// FP32-mixed, 852 against 1135, 1155 and 793 us FP64; the 8x8x8 tiles gain in
+// FP64 from some 16 k octs on (27 k octs: 73.8 against 75.8 us, 9 k octs:
+// 36.9 against 34.8). A few hundred octs take one tile's latency, 14-18 us,
+// in any shape.
 int default_shape(const rb_context* c, int l, const Level& L) {
-  int s = 0;                                            // single oct
-  if (L.complete && L.noct >= 64 * 148) s = 4;          // 8x8x8 cells
-  else if (L.noct >= 8 * 64) s = 1;                     // 4x4x4 cells
-  return shape_fits(c, l, s) ? s : 0;
+  if (c->precision == RB_PREC_FP64 && L.noct >= 16384 && shape_fits(c, l, 4)) return 4;
+  for (int s : {3, 1})
+    if (shape_fits(c, l, s)) return s;
+  return 0;
 }
 
 // Device cell of nbor(igrid,j), j = 1..6, for the level's octs in active

@@ -65,142 +65,6 @@ struct S2Geom {
   static_assert(RAW_BYTES % 16 == 0 && Q4_BYTES % 16 == 0 && QP_BYTES % 16 == 0, "16-byte aligned sections");
 };
 
-// Half slope dq/2 of one variable in one direction (uslope, umuscl.f90:1241-1327):
-// ST = 1 minmod, ST = 2 moncen, in FP32 with the sign applied last.
-template <int ST>
-__device__ __forceinline__ float hslope(float qm1, float q0, float qp1) {
-  const float a = q0 - qm1, b = qp1 - q0;
-  const float m = fminf(fabsf(a), fabsf(b));
-  float s;
-  if (ST == 1) {
-    s = copysignf(0.5f * m, a);
-  } else {
-    const float t = a + b;
-    s = copysignf(fminf(m, 0.25f * fabsf(t)), t);
-  }
-  return a * b <= 0.0f ? 0.0f : s;
-}
-
-// Half slope from the two one-sided differences a = q0 - q(-1), b = q(+1) - q0.
-template <int ST>
-__device__ __forceinline__ float hslope_ab(float a, float b) {
-  const float m = fminf(fabsf(a), fabsf(b));
-  float s;
-  if (ST == 1) {
-    s = copysignf(0.5f * m, a);
-  } else {
-    const float t = a + b;
-    s = copysignf(fminf(m, 0.25f * fabsf(t)), t);
-  }
-  return a * b <= 0.0f ? 0.0f : s;
-}
-
-// ctoprim (umuscl.f90:861-965) for the FP32-mixed kernels. The density
-// floor, the internal energy E - |m|^2/(2 rho) and the pressure floor are
-// FP64; the reciprocal of rho is the FP32 one refined by one Newton step in
-// FP64, and the velocities are FP32. With
-// P = (gamma-1) rho max(E/rho - v^2/2, smalle) and
-// smalle = smallc^2/gamma/(gamma-1): P = max((gamma-1)(E - |m|^2/(2 rho)), rho smallc^2/gamma).
-__device__ __forceinline__ Prim<float> ctoprim_mixed(const double u[5], double smallr, double gm1, double pfc) {
-  const double rho = fmax(u[0], smallr);
-  const float rf = (float)rho;
-  const float irf = __fdividef(1.0f, rf);
-  const double ir = fma((double)irf, fma(-rho, (double)irf, 1.0), (double)irf);
-  const double ke = u[1] * u[1] + u[2] * u[2] + u[3] * u[3];
-  const double p = fmax(gm1 * fma(-0.5 * ke, ir, u[4]), pfc * rho);
-  Prim<float> q;
-  q.r = rf;
-  q.u = (float)u[1] * irf;
-  q.v = (float)u[2] * irf;
-  q.w = (float)u[3] * irf;
-  q.p = (float)p;
-  return q;
-}
-
-// HLLC flux (riemann_hllc, godunov_utils.f90:988-1209) in FP32 for the mixed
-// path, times dt/dx. Face frame (rho, u_n, P, u_t1, u_t2) in, flux of (mass,
-// normal momentum, energy, t1 momentum, t2 momentum) out. The larger of the
-// two fast sound speeds is formed with one reciprocal and one square root,
-// and the sampled state's side is chosen before its energy is formed.
-__device__ __forceinline__ void hllc_f32(const float ql[5], const float qr[5], const Consts<float>& c,
-                                         float smallc2, float dtdx, float f[5]) {
-  const float rl = fmaxf(ql[0], c.smallr), ul = ql[1], Pl = fmaxf(ql[2], rl * c.smallp);
-  const float rr = fmaxf(qr[0], c.smallr), ur = qr[1], Pr = fmaxf(qr[2], rr * c.smallp);
-  // max(gamma Pl/rl, gamma Pr/rr, smallc^2), rl, rr > 0
-  const float a2 = fmaxf(fmaxf(Pl * rr, Pr * rl) * (c.gamma * __fdividef(1.0f, rl * rr)), smallc2);
-  const float cmax = sqrtf(a2);
-  const float SL = fminf(ul, ur) - cmax, SR = fmaxf(ul, ur) + cmax;
-  const float rcl = rl * (ul - SL), rcr = rr * (SR - ur);
-  const float inv = __fdividef(1.0f, rcr + rcl);
-  const float ustar = (rcr * ur + rcl * ul + (Pl - Pr)) * inv;
-  const float Pstar = (rcr * Pl + rcl * Pr + rcl * rcr * (ul - ur)) * inv;
-  // sampling at x/t = 0: outer left if SL > 0, left star if ustar > 0, right
-  // star if SR > 0, else outer right
-  const bool outl = SL > 0.0f, lft = ustar > 0.0f;
-  const bool side = outl || lft;
-  const bool star = !outl && (lft || SR > 0.0f);
-  const float rs = side ? rl : rr, us = side ? ul : ur, Ss = side ? SL : SR, Ps = side ? Pl : Pr;
-  const float t1 = side ? ql[3] : qr[3], t2 = side ? ql[4] : qr[4];
-  const float num = Ss - us, iden = __fdividef(1.0f, Ss - ustar);
-  const float ratio = star ? num * iden : 1.0f;
-  const float ro = rs * ratio;
-  const float uo = star ? ustar : us;
-  const float Po = star ? Pstar : Ps;
-  const float ets = Ps * c.entho + 0.5f * rs * (us * us + t1 * t1 + t2 * t2);
-  const float eto = star ? (num * ets - Ps * us + Pstar * ustar) * iden : ets;
-  const float uos = uo * dtdx;
-  const float mo = ro * uos;
-  f[0] = mo;
-  f[1] = mo * uo + Po * dtdx;
-  f[2] = (eto + Po) * uos;
-  f[3] = mo * t1;
-  f[4] = mo * t2;
-}
-
-// MUSCL-Hancock half-step state of a cell for the FP32 path: h = q + s dt/(2dx)
-// with the source terms of trace3d (umuscl.f90:576-580), equal in every
-// direction on a cubic cell. hd[v][d] are half slopes; th = dt/dx (the factor
-// 1/2 of the half step cancels the 2 of the full slope).
-__device__ __forceinline__ void half_step(const Prim<float>& q, const float hd[5][3], float gamma, float th,
-                                          float h[5]) {
-  const float r = q.r, u = q.u, v = q.v, w = q.w, p = q.p;
-  const float divv = hd[1][0] + hd[2][1] + hd[3][2];
-  const float ir = __fdividef(1.0f, r);
-  h[0] = r - th * (u * hd[0][0] + v * hd[0][1] + w * hd[0][2] + divv * r);
-  h[4] = p - th * (u * hd[4][0] + v * hd[4][1] + w * hd[4][2] + divv * (gamma * p));
-  h[1] = u - th * (u * hd[1][0] + v * hd[1][1] + w * hd[1][2] + hd[4][0] * ir);
-  h[2] = v - th * (u * hd[2][0] + v * hd[2][1] + w * hd[2][2] + hd[4][1] * ir);
-  h[3] = w - th * (u * hd[3][0] + v * hd[3][1] + w * hd[3][2] + hd[4][2] * ir);
-}
-
-// face states of direction d: right state at the lower face P = h - hd,
-// left state at the upper face M = h + hd, density floored to the cell's
-// (trace3d: if (q < smallr) q = r)
-__device__ __forceinline__ void face_pair(const float h[5], const float hd[5][3], int d, float r, float smallr,
-                                          float P[5], float M[5]) {
-#pragma unroll
-  for (int v = 0; v < 5; v++) { P[v] = h[v] - hd[v][d]; M[v] = h[v] + hd[v][d]; }
-  if (P[0] < smallr) P[0] = r;
-  if (M[0] < smallr) M[0] = r;
-}
-
-// (rho, u, v, w, p) -> face frame of direction d (cmpflxm's permutation)
-__device__ __forceinline__ void face_frame(const float s[5], int d, float o[5]) {
-  o[0] = s[0];
-  o[2] = s[4];
-  if (d == 0) { o[1] = s[1]; o[3] = s[2]; o[4] = s[3]; }
-  else if (d == 1) { o[1] = s[2]; o[3] = s[1]; o[4] = s[3]; }
-  else { o[1] = s[3]; o[3] = s[1]; o[4] = s[2]; }
-}
-// face-frame flux -> (rho, mx, my, mz, E)
-__device__ __forceinline__ void flux_back(const float f[5], int d, float o[5]) {
-  o[0] = f[0];
-  o[4] = f[2];
-  if (d == 0) { o[1] = f[1]; o[2] = f[3]; o[3] = f[4]; }
-  else if (d == 1) { o[2] = f[1]; o[1] = f[3]; o[3] = f[4]; }
-  else { o[3] = f[1]; o[1] = f[3]; o[2] = f[4]; }
-}
-
 // One work item (TX x TY column, z range [z0, z0+hz)) of one problem.
 template <int TX, int TY, int ST>
 __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int item) {

@@ -21,11 +21,11 @@ struct TileShape {
 // Supported tile shapes, indexed by shape id.
 constexpr int kNumTileShapes = 5;
 constexpr TileShape kTileShapes[kNumTileShapes] = {
-    {2, 2, 2, 64},    // one oct: the reference's per-oct stencil
-    {4, 4, 4, 128},
-    {8, 4, 4, 256},
+    {2, 2, 2, 32},    // one oct: the reference's per-oct stencil
+    {4, 4, 4, 64},
+    {8, 4, 4, 128},
     {8, 8, 4, 256},
-    {8, 8, 8, 256},
+    {8, 8, 8, 512},
 };
 
 size_t tile_smem_f64(int shape);

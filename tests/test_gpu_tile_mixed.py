@@ -1,0 +1,40 @@
+"""GPU: the FP32-mixed oct-tile kernel in every tile shape: the shapes give the
+same bits (each cell and face is one function of its stencil, whichever tile
+computes it), and the state stays within FP32 rounding of the FP64 path."""
+import numpy as np
+import pytest
+
+from ramses_b200 import runtime
+
+from helpers import sedov_amr
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("pressure_fix", [False, True])
+@pytest.mark.parametrize("slope_type,riemann", [(1, "hllc"), (2, "hllc"), (3, "hllc"), (2, "llf")])
+@pytest.mark.parametrize("levels", [(2, 4), (3, 5)])
+def test_shapes_identical_and_close_to_fp64(cuda_lib, levels, slope_type, riemann, pressure_fix):
+    tree, hp, u = sedov_amr(*levels, slope_type=slope_type, riemann=riemann)
+    hp.pressure_fix, hp.beta_fix = pressure_fix, 10.0 if pressure_fix else 0.0
+    u = u.copy()
+    rng = np.random.default_rng(5)
+    u[0] *= 1.0 + 0.2 * rng.random(u.shape[1])
+    u[1:4] += 0.1 * u[0] * (rng.random((3, u.shape[1])) - 0.5)
+    u[4] += 0.5 * (u[1:4] ** 2).sum(0) / np.maximum(u[0], 1e-10) + 0.05
+    outs = []
+    for shape in range(5):
+        with runtime.Solver(tree, hp, precision="mixed", uold=u) as s:
+            for l in range(tree.levelmin, tree.nlevelmax + 1):
+                s.set_tile_shape(l, shape)
+            s.run(max_steps=2)
+            outs.append(s.download_state())
+    for o in outs[1:]:
+        np.testing.assert_array_equal(outs[0], o)
+    with runtime.Solver(tree, hp, uold=u) as s:
+        s.run(max_steps=2)
+        ref = s.download_state()
+    # a few hundred FP32 roundings (6e-8 each) per cell over the steps of two
+    # coarse steps, amplified by at most the limiter's switch: 1e-5 of the norm
+    for v in range(5):
+        assert np.linalg.norm(outs[0][v] - ref[v]) <= 1e-5 * np.linalg.norm(ref[v]), v
