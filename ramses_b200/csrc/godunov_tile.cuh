@@ -209,7 +209,7 @@ __device__ __forceinline__ void trace_slot(const States<R>& q, int s, const Cons
   using G = TileGeom<TX, TY, TZ>;
   constexpr int st[3] = {1, G::SX, G::SX * G::SY};
   const Prim<R> q0 = q.get(s);
-  if constexpr (sizeof(R) == 4 && RS == RB_RIEMANN_HLLC && (ST == 1 || ST == 2)) {
+  if constexpr (sizeof(R) == 4 && RS != 0 && (ST == 1 || ST == 2)) {
     float hd[5][3], h[5];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
@@ -415,42 +415,56 @@ __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_con
   const int fx0 = x + (TX + 1) * (y + TY * z);
   const int fy0 = NFX + x + TX * (y + (TY + 1) * z);
   const int fz0 = NFX + NFY + x + TX * (y + TY * z);
-  Prim<R> P[3];
-  if (code_own != -1) {
-    Prim<R> sm[3];
-    trace_slot<R, TX, TY, TZ, RS, ST>(q, s_own, c, slope_type, dtd, 7u, P, sm);
-    Ls.put(fx0 + 1, sm[0]);
-    Ls.put(fy0 + TX, sm[1]);
-    Ls.put(fz0 + TX * TY, sm[2]);
-  }
   // present(s): the tile-interior cell belongs to an oct of this level
   // (its update and its faces are used; bit 1 of okf). A block coded -1 is
   // absent and not a stencil source of any present oct, so no face touching
   // it is used.
-#pragma unroll 1
-  for (int it = tid; it < G::NSLAB; it += NT) {
-    const int side = it >= G::NU, r = side ? it - G::NU : it;
-    int s, d, f;  // slab slot, direction, face towards the tile
-    if (r < G::NUX) {
-      const int yy = r % TY, zz = r / TY;
-      d = 0; s = (side ? TX + 2 : 1) + SX * ((yy + 2) + SY * (zz + 2)); f = (TX + 1) * (yy + TY * zz);
-    } else if (r < G::NUX + G::NUY) {
-      const int k = r - G::NUX, xx = k % TX, zz = k / TX;
-      d = 1; s = (xx + 2) + SX * ((side ? TY + 2 : 1) + SY * (zz + 2)); f = NFX + xx + TX * (TY + 1) * zz;
-    } else {
-      const int k = r - G::NUX - G::NUY, xx = k % TX, yy = k / TX;
-      d = 2; s = (xx + 2) + SX * ((yy + 2) + SY * (side ? TZ + 2 : 1)); f = NFX + NFY + xx + TX * yy;
+  // A face on a tile's side is solved by both tiles and must get one flux.
+  // FP64 code is never contracted and the FP32 forms of hydro_core.cuh spell
+  // their contraction out, so any copy of them rounds alike; the other FP32
+  // schemes go through one instance of the trace (own cell j = 0, then the
+  // slab cells) and one of the solver per direction, as loops that are not
+  // unrolled (9 % of a Sedov run where it is not needed).
+  constexpr bool kOneSite = sizeof(R) == 4 && !(RS != 0 && (ST == 1 || ST == 2));
+  Prim<R> P[3];
+  constexpr int NJ = 1 + (G::NSLAB + NT - 1) / NT;
+#pragma unroll (kOneSite ? 1 : 2)
+  for (int j = 0; j < NJ; j++) {
+    int s = s_own, d = 0, f = 0, r = 0, side = 0;  // slab: slot, direction, face towards the tile
+    bool live = code_own != -1;
+    unsigned mask = 7u;
+    if (j > 0) {
+      const int it = tid + (j - 1) * NT;
+      if (it >= G::NSLAB) break;
+      side = it >= G::NU; r = side ? it - G::NU : it;
+      if (r < G::NUX) {
+        const int yy = r % TY, zz = r / TY;
+        d = 0; s = (side ? TX + 2 : 1) + SX * ((yy + 2) + SY * (zz + 2)); f = (TX + 1) * (yy + TY * zz);
+      } else if (r < G::NUX + G::NUY) {
+        const int k = r - G::NUX, xx = k % TX, zz = k / TX;
+        d = 1; s = (xx + 2) + SX * ((side ? TY + 2 : 1) + SY * (zz + 2)); f = NFX + xx + TX * (TY + 1) * zz;
+      } else {
+        const int k = r - G::NUX - G::NUY, xx = k % TX, yy = k / TX;
+        d = 2; s = (xx + 2) + SX * ((yy + 2) + SY * (side ? TZ + 2 : 1)); f = NFX + NFY + xx + TX * yy;
+      }
+      const int step = d == 0 ? 1 : d == 1 ? SX : SX * SY;
+      live = (okf[side ? s - step : s + step] & 2) != 0;
+      mask = 1u << d;
     }
-    const int step = d == 0 ? 1 : d == 1 ? SX : SX * SY;
-    if (!(okf[side ? s - step : s + step] & 2)) continue;
+    if (!live) continue;
     Prim<R> sp[3], sm[3];
-    trace_slot<R, TX, TY, TZ, RS, ST>(q, s, c, slope_type, dtd, 1u << d, sp, sm);
-    // lower slab: the left state of its face; upper slab: the right state
-    if (side) {
+    trace_slot<R, TX, TY, TZ, RS, ST>(q, s, c, slope_type, dtd, mask, sp, sm);
+    if (j == 0) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) P[k] = sp[k];
+      Ls.put(fx0 + 1, sm[0]);
+      Ls.put(fy0 + TX, sm[1]);
+      Ls.put(fz0 + TX * TY, sm[2]);
+    } else if (side) {  // upper slab: the right state of its face
       if (d == 0) Us.put(r, sp[0]);
       else if (d == 1) Us.put(r, sp[1]);
       else Us.put(r, sp[2]);
-    } else {
+    } else {            // lower slab: the left state
       if (d == 0) Ls.put(f, sm[0]);
       else if (d == 1) Ls.put(f, sm[1]);
       else Ls.put(f, sm[2]);
@@ -523,8 +537,8 @@ __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_con
     R ql[5], qr[5], fg[6], fo[5];
     to_face(L, D, ql);
     to_face(Rr, D, qr);
-    if constexpr (sizeof(R) == 4 && RS == RB_RIEMANN_HLLC && (ST == 1 || ST == 2)) {
-      hllc_f32<PF>(ql, qr, c, smallc2, dtdx, fg);
+    if constexpr (sizeof(R) == 4 && RS != 0 && (ST == 1 || ST == 2)) {
+      riemann_f32<RS, PF>(ql, qr, c, smallc2, dtdx, fg);
       from_face(fg, D, fo);
       if (PF) tmp[1] = zero_face ? (R)0 : fg[5];
     } else {
@@ -575,34 +589,55 @@ __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_con
       Ls.at(f, 1) = tmp[1];
     }
   };
-  // a face is used only when one of its two cells is a present cell
+  // Per direction: the lower face of the own cell (j = 0), then the far faces,
+  // whose three groups go to different threads. A face is used only when one
+  // of its two cells is a present cell.
   Prim<R> flo[3];    // fluxes through the own cell's lower faces
   R tlo[3][2] = {{(R)0, (R)0}, {(R)0, (R)0}, {(R)0, (R)0}};
-  if (own) {
-    const int fo_ = okf[s_own];
-    const int fl0 = fo_ | okf[s_own - 1], fl1 = fo_ | okf[s_own - SX], fl2 = fo_ | okf[s_own - SX * SY];
-    if (fl0 & 2) face_flux(std::integral_constant<int, 0>(), fx0, x, y, z, Ls.get(fx0), P[0], fl0, flo[0], tlo[0]);
-    if (fl1 & 2) face_flux(std::integral_constant<int, 1>(), fy0, x, y, z, Ls.get(fy0), P[1], fl1, flo[1], tlo[1]);
-    if (fl2 & 2) face_flux(std::integral_constant<int, 2>(), fz0, x, y, z, Ls.get(fz0), P[2], fl2, flo[2], tlo[2]);
-  }
-  // the tile's far faces
+  auto dir_faces = [&](auto dir, int f_own, int j0, int j1, int r0, int nu, int n1) {
+    constexpr int D = decltype(dir)::value;
+    constexpr int step = D == 0 ? 1 : D == 1 ? SX : SX * SY;
+    // the far faces' threads start at r0 modulo the block, so that the three
+    // directions load different warps
 #pragma unroll 1
-  for (int r = tid; r < G::NU; r += NT) {
-    Prim<R> fo;
-    R t[2];
-    if (r < G::NUX) {
-      const int yy = r % TY, zz = r / TY, s = (TX + 2) + SX * ((yy + 2) + SY * (zz + 2));
-      const int f = TX + (TX + 1) * (yy + TY * zz), fl = okf[s - 1] | okf[s];
-      if (fl & 2) face_flux(std::integral_constant<int, 0>(), f, TX, yy, zz, Ls.get(f), Us.get(r), fl, fo, t);
-    } else if (r < G::NUX + G::NUY) {
-      const int k = r - G::NUX, xx = k % TX, zz = k / TX, s = (xx + 2) + SX * ((TY + 2) + SY * (zz + 2));
-      const int f = NFX + xx + TX * (TY + (TY + 1) * zz), fl = okf[s - SX] | okf[s];
-      if (fl & 2) face_flux(std::integral_constant<int, 1>(), f, xx, TY, zz, Ls.get(f), Us.get(r), fl, fo, t);
-    } else {
-      const int k = r - G::NUX - G::NUY, xx = k % TX, yy = k / TX, s = (xx + 2) + SX * ((yy + 2) + SY * (TZ + 2));
-      const int f = NFX + NFY + xx + TX * (yy + TY * TZ), fl = okf[s - SX * SY] | okf[s];
-      if (fl & 2) face_flux(std::integral_constant<int, 2>(), f, xx, yy, TZ, Ls.get(f), Us.get(r), fl, fo, t);
+    for (int j = j0; j < j1; j++) {
+      int f = f_own, cx = x, cy = y, cz = z, r = 0;
+      if (j == 0) {
+        if (!own) continue;
+      } else {
+        r = (tid + NT - r0 % NT) % NT + (j - 1) * NT;
+        if (r >= nu) break;
+        const int k0 = r % n1, k1 = r / n1;
+        if (D == 0) { cx = TX; cy = k0; cz = k1; f = TX + (TX + 1) * (cy + TY * cz); }
+        else if (D == 1) { cx = k0; cy = TY; cz = k1; f = NFX + cx + TX * (TY + (TY + 1) * cz); }
+        else { cx = k0; cy = k1; cz = TZ; f = NFX + NFY + cx + TX * (cy + TY * TZ); }
+      }
+      const int s = (cx + 2) + SX * ((cy + 2) + SY * (cz + 2));
+      const int fl = okf[s] | okf[s - step];
+      if (!(fl & 2)) continue;
+      Prim<R> fo;
+      R t[2];
+      face_flux(dir, f, cx, cy, cz, Ls.get(f), j == 0 ? P[D] : Us.get(r0 + r), fl, fo, t);
+      if (j == 0) {
+        flo[D] = fo;
+        if (PF) { tlo[D][0] = t[0]; tlo[D][1] = t[1]; }
+      }
     }
+  };
+  // the passes [j0, j1) of every direction
+  auto faces = [&](int j0, int j1) {
+    constexpr std::integral_constant<int, 0> DX{};
+    constexpr std::integral_constant<int, 1> DY{};
+    constexpr std::integral_constant<int, 2> DZ{};
+    dir_faces(DX, fx0, j0, min(j1, 1 + (G::NUX + NT - 1) / NT), 0, G::NUX, TY);
+    dir_faces(DY, fy0, j0, min(j1, 1 + (G::NUY + NT - 1) / NT), G::NUX, G::NUY, TX);
+    dir_faces(DZ, fz0, j0, min(j1, 1 + (G::NUZ + NT - 1) / NT), G::NUX + G::NUY, G::NUZ, TX);
+  };
+  if constexpr (kOneSite) {
+    faces(0, 1 << 20);
+  } else {
+    faces(0, 1);        // straight-line code: the three solves overlap
+    faces(1, 1 << 20);
   }
   cp_async_wait<0>();  // this thread's correction entries (E)
   __syncthreads();

@@ -690,8 +690,12 @@ __device__ __forceinline__ void from_face(const R f[6], int d, R out[5]) {
 }
 
 // ---------------------------------------------------------------------------
-// FP32-mixed forms for HLLC with minmod (ST = 1) or moncen (ST = 2) slopes and
-// the MUSCL-Hancock predictor, in half slopes.
+// FP32-mixed forms for minmod (ST = 1) or moncen (ST = 2) slopes and the
+// MUSCL-Hancock predictor, in half slopes. A face at the edge of a tile or
+// column is solved by two CTAs, and often by two inlined copies of this code:
+// the products and sums are written with the contraction spelled out (fmaf,
+// __fmul_rn, __fadd_rn), so that every copy rounds alike and the face has one
+// flux (the FP64 accumulation of the fluxes then telescopes).
 // ---------------------------------------------------------------------------
 // Half slope dq/2 of one variable in one direction (uslope, umuscl.f90:1241-1327):
 // ST = 1 minmod, ST = 2 moncen, in FP32 with the sign applied last.
@@ -753,16 +757,18 @@ __device__ __forceinline__ Prim<float> ctoprim_mixed(const double u[5], double s
 template <bool THERMAL = false>
 __device__ __forceinline__ void hllc_f32(const float ql[5], const float qr[5], const Consts<float>& c,
                                          float smallc2, float dtdx, float* f) {
-  const float rl = fmaxf(ql[0], c.smallr), ul = ql[1], Pl = fmaxf(ql[2], rl * c.smallp);
-  const float rr = fmaxf(qr[0], c.smallr), ur = qr[1], Pr = fmaxf(qr[2], rr * c.smallp);
+  const float rl = fmaxf(ql[0], c.smallr), ul = ql[1], Pl = fmaxf(ql[2], __fmul_rn(rl, c.smallp));
+  const float rr = fmaxf(qr[0], c.smallr), ur = qr[1], Pr = fmaxf(qr[2], __fmul_rn(rr, c.smallp));
   // max(gamma Pl/rl, gamma Pr/rr, smallc^2), rl, rr > 0
-  const float a2 = fmaxf(c.gamma * fmaxf(Pl * __fdividef(1.0f, rl), Pr * __fdividef(1.0f, rr)), smallc2);
+  const float a2 = fmaxf(
+      __fmul_rn(c.gamma, fmaxf(__fmul_rn(Pl, __fdividef(1.0f, rl)), __fmul_rn(Pr, __fdividef(1.0f, rr)))), smallc2);
   const float cmax = sqrtf(a2);
-  const float SL = fminf(ul, ur) - cmax, SR = fmaxf(ul, ur) + cmax;
-  const float rcl = rl * (ul - SL), rcr = rr * (SR - ur);
-  const float inv = __fdividef(1.0f, rcr + rcl);
-  const float ustar = (rcr * ur + rcl * ul + (Pl - Pr)) * inv;
-  const float Pstar = (rcr * Pl + rcl * Pr + rcl * rcr * (ul - ur)) * inv;
+  const float SL = __fsub_rn(fminf(ul, ur), cmax), SR = __fadd_rn(fmaxf(ul, ur), cmax);
+  const float rcl = __fmul_rn(rl, __fsub_rn(ul, SL)), rcr = __fmul_rn(rr, __fsub_rn(SR, ur));
+  const float inv = __fdividef(1.0f, __fadd_rn(rcr, rcl));
+  const float ustar = __fmul_rn(fmaf(rcr, ur, fmaf(rcl, ul, __fsub_rn(Pl, Pr))), inv);
+  const float Pstar =
+      __fmul_rn(fmaf(rcr, Pl, fmaf(rcl, Pr, __fmul_rn(__fmul_rn(rcl, rcr), __fsub_rn(ul, ur)))), inv);
   // sampling at x/t = 0: outer left if SL > 0, left star if ustar > 0, right
   // star if SR > 0, else outer right
   const bool outl = SL > 0.0f, lft = ustar > 0.0f;
@@ -770,22 +776,74 @@ __device__ __forceinline__ void hllc_f32(const float ql[5], const float qr[5], c
   const bool star = !outl && (lft || SR > 0.0f);
   const float rs = side ? rl : rr, us = side ? ul : ur, Ss = side ? SL : SR, Ps = side ? Pl : Pr;
   const float t1 = side ? ql[3] : qr[3], t2 = side ? ql[4] : qr[4];
-  const float num = Ss - us, iden = __fdividef(1.0f, Ss - ustar);
-  const float ratio = star ? num * iden : 1.0f;
-  const float ro = rs * ratio;
+  const float num = __fsub_rn(Ss, us), iden = __fdividef(1.0f, __fsub_rn(Ss, ustar));
+  const float ratio = star ? __fmul_rn(num, iden) : 1.0f;
+  const float ro = __fmul_rn(rs, ratio);
   const float uo = star ? ustar : us;
   const float Po = star ? Pstar : Ps;
-  const float es = Ps * c.entho;
-  const float ets = es + 0.5f * rs * (us * us + t1 * t1 + t2 * t2);
-  const float eto = star ? (num * ets - Ps * us + Pstar * ustar) * iden : ets;
-  const float uos = uo * dtdx;
-  const float mo = ro * uos;
+  const float es = __fmul_rn(Ps, c.entho);
+  const float ets = fmaf(__fmul_rn(0.5f, rs), fmaf(us, us, fmaf(t1, t1, __fmul_rn(t2, t2))), es);
+  const float eto =
+      star ? __fmul_rn(fmaf(num, ets, fmaf(Pstar, ustar, -__fmul_rn(Ps, us))), iden) : ets;
+  const float uos = __fmul_rn(uo, dtdx);
+  const float mo = __fmul_rn(ro, uos);
   f[0] = mo;
-  f[1] = mo * uo + Po * dtdx;
-  f[2] = (eto + Po) * uos;
-  f[3] = mo * t1;
-  f[4] = mo * t2;
-  if (THERMAL) f[5] = es * ratio * uos;
+  f[1] = fmaf(mo, uo, __fmul_rn(Po, dtdx));
+  f[2] = __fmul_rn(__fadd_rn(eto, Po), uos);
+  f[3] = __fmul_rn(mo, t1);
+  f[4] = __fmul_rn(mo, t2);
+  if (THERMAL) f[5] = __fmul_rn(__fmul_rn(es, ratio), uos);
+}
+
+// llf (RS = RB_RIEMANN_LLF, godunov_utils.f90:660-820) and hll (:825-983), as hllc_f32.
+template <int RS, bool THERMAL>
+__device__ __forceinline__ void llf_hll_f32(const float ql[5], const float qr[5], const Consts<float>& c,
+                                            float dtdx, float* f) {
+  const float rl = fmaxf(ql[0], c.smallr), pl = fmaxf(ql[2], __fmul_rn(rl, c.smallp));
+  const float rr = fmaxf(qr[0], c.smallr), pr = fmaxf(qr[2], __fmul_rn(rr, c.smallp));
+  const float cl2 = __fmul_rn(__fmul_rn(c.gamma, pl), __fdividef(1.0f, rl));
+  const float cr2 = __fmul_rn(__fmul_rn(c.gamma, pr), __fdividef(1.0f, rr));
+  float uL[6], uR[6], fL[6], fR[6];
+  auto cons_flux = [&](const float q[5], float u[6], float fl[6]) {
+    const float k = fmaf(q[1], q[1], fmaf(q[3], q[3], __fmul_rn(q[4], q[4])));
+    u[5] = __fmul_rn(q[2], c.entho);
+    u[0] = q[0];
+    u[1] = __fmul_rn(q[0], q[1]);
+    u[2] = fmaf(__fmul_rn(0.5f, q[0]), k, u[5]);
+    u[3] = __fmul_rn(q[0], q[3]);
+    u[4] = __fmul_rn(q[0], q[4]);
+    fl[0] = u[1];
+    fl[1] = fmaf(u[1], q[1], q[2]);
+    fl[2] = __fmul_rn(q[1], __fadd_rn(u[2], q[2]));
+    fl[3] = __fmul_rn(q[1], u[3]);
+    fl[4] = __fmul_rn(q[1], u[4]);
+    fl[5] = __fmul_rn(q[1], u[5]);
+  };
+  cons_flux(ql, uL, fL);
+  cons_flux(qr, uR, fR);
+  if (RS == RB_RIEMANN_LLF) {
+    const float cmax = fmaxf(__fadd_rn(fabsf(ql[1]), sqrtf(cl2)), __fadd_rn(fabsf(qr[1]), sqrtf(cr2)));
+    const float h = __fmul_rn(0.5f, dtdx);
+#pragma unroll
+    for (int n = 0; n < (THERMAL ? 6 : 5); n++)
+      f[n] = __fmul_rn(fmaf(-cmax, __fsub_rn(uR[n], uL[n]), __fadd_rn(fL[n], fR[n])), h);
+  } else {
+    const float cm = sqrtf(fmaxf(cl2, cr2));
+    const float SL = fminf(__fsub_rn(fminf(ql[1], qr[1]), cm), 0.0f);
+    const float SR = fmaxf(__fadd_rn(fmaxf(ql[1], qr[1]), cm), 0.0f);
+    const float SS = __fmul_rn(SR, SL), h = __fdividef(dtdx, __fsub_rn(SR, SL));
+#pragma unroll
+    for (int n = 0; n < (THERMAL ? 6 : 5); n++)
+      f[n] = __fmul_rn(fmaf(SR, fL[n], fmaf(-SL, fR[n], __fmul_rn(SS, __fsub_rn(uR[n], uL[n])))), h);
+  }
+}
+
+// The solver RS (llf, hll, hllc) for the FP32 path, times dt/dx, as hllc_f32.
+template <int RS, bool THERMAL = false>
+__device__ __forceinline__ void riemann_f32(const float ql[5], const float qr[5], const Consts<float>& c,
+                                            float smallc2, float dtdx, float* f) {
+  if constexpr (RS == RB_RIEMANN_HLLC) hllc_f32<THERMAL>(ql, qr, c, smallc2, dtdx, f);
+  else llf_hll_f32<RS, THERMAL>(ql, qr, c, dtdx, f);
 }
 
 // MUSCL-Hancock half-step state of a cell for the FP32 path: h = q + s dt/(2dx)
@@ -795,13 +853,17 @@ __device__ __forceinline__ void hllc_f32(const float ql[5], const float qr[5], c
 __device__ __forceinline__ void half_step(const Prim<float>& q, const float hd[5][3], float gamma, float th,
                                           float h[5]) {
   const float r = q.r, u = q.u, v = q.v, w = q.w, p = q.p;
-  const float divv = hd[1][0] + hd[2][1] + hd[3][2];
+  const float divv = __fadd_rn(__fadd_rn(hd[1][0], hd[2][1]), hd[3][2]);
   const float ir = __fdividef(1.0f, r);
-  h[0] = r - th * (u * hd[0][0] + v * hd[0][1] + w * hd[0][2] + divv * r);
-  h[4] = p - th * (u * hd[4][0] + v * hd[4][1] + w * hd[4][2] + divv * (gamma * p));
-  h[1] = u - th * (u * hd[1][0] + v * hd[1][1] + w * hd[1][2] + hd[4][0] * ir);
-  h[2] = v - th * (u * hd[2][0] + v * hd[2][1] + w * hd[2][2] + hd[4][1] * ir);
-  h[3] = w - th * (u * hd[3][0] + v * hd[3][1] + w * hd[3][2] + hd[4][2] * ir);
+  // -th (u . grad q + x y) + q
+  auto step = [&](float qv, const float g[3], float x, float y) {
+    return fmaf(-th, fmaf(x, y, fmaf(w, g[2], fmaf(v, g[1], __fmul_rn(u, g[0])))), qv);
+  };
+  h[0] = step(r, hd[0], divv, r);
+  h[4] = step(p, hd[4], divv, __fmul_rn(gamma, p));
+  h[1] = step(u, hd[1], hd[4][0], ir);
+  h[2] = step(v, hd[2], hd[4][1], ir);
+  h[3] = step(w, hd[3], hd[4][2], ir);
 }
 
 // face states of direction d: right state at the lower face P = h - hd,
@@ -810,7 +872,7 @@ __device__ __forceinline__ void half_step(const Prim<float>& q, const float hd[5
 __device__ __forceinline__ void face_pair(const float h[5], const float hd[5][3], int d, float r, float smallr,
                                           float P[5], float M[5]) {
 #pragma unroll
-  for (int v = 0; v < 5; v++) { P[v] = h[v] - hd[v][d]; M[v] = h[v] + hd[v][d]; }
+  for (int v = 0; v < 5; v++) { P[v] = __fsub_rn(h[v], hd[v][d]); M[v] = __fadd_rn(h[v], hd[v][d]); }
   if (P[0] < smallr) P[0] = r;
   if (M[0] < smallr) M[0] = r;
 }

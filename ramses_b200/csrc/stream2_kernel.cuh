@@ -21,8 +21,8 @@
 // (cp.async, one plane of prefetch distance) keeps the CTA at ~70 KB, three
 // CTAs per SM.
 //
-// HLLC with minmod (ST = 1) or moncen (ST = 2) slopes, MUSCL-Hancock
-// predictor; other schemes and the FP64 drop-in use stream_kernel.cuh.
+// llf, hll or hllc (RS) with minmod (ST = 1) or moncen (ST = 2) slopes,
+// MUSCL-Hancock predictor; other schemes and the FP64 drop-in use stream_kernel.cuh.
 // References: ctoprim umuscl.f90:861-965, uslope :1241-1327, trace3d
 // :483-708, cmpflxm :714-856, riemann_hllc godunov_utils.f90:988-1209,
 // update godunov_fine.f90:751-792, cmpdt godunov_utils.f90:5-120.
@@ -66,7 +66,7 @@ struct S2Geom {
 };
 
 // One work item (TX x TY column, z range [z0, z0+hz)) of one problem.
-template <int TX, int TY, int ST>
+template <int TX, int TY, int RS, int ST>
 __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int item) {
   using G = S2Geom<TX, TY>;
   constexpr int SX = G::SX, SY = G::SY, NS = G::NS, SXP = G::SXP, NQS = G::NQS, CX = G::CX, NIN = G::NIN;
@@ -255,7 +255,7 @@ __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int
         float ql[5], qr[5], ff[5], fo[5];
         face_frame(L, 0, ql);
         face_frame(R, 0, qr);
-        hllc_f32(ql, qr, c, smallc2, dtdx, ff);
+        riemann_f32<RS>(ql, qr, c, smallc2, dtdx, ff);
         flux_back(ff, 0, fo);
         fx4[slot] = make_float4(fo[0], fo[1], fo[2], fo[3]);
         fx1[slot] = fo[4];
@@ -264,7 +264,7 @@ __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int
         float ql[5], qr[5], ff[5], fo[5];
         face_frame(qmz, 2, ql);
         face_frame(zP, 2, qr);
-        hllc_f32(ql, qr, c, smallc2, dtdx, ff);
+        riemann_f32<RS>(ql, qr, c, smallc2, dtdx, ff);
         flux_back(ff, 2, fo);
 #pragma unroll
         for (int v = 0; v < 5; v++) fzd[v] = (double)fo[v];
@@ -290,7 +290,7 @@ __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int
           float ql[5], qr[5], ff[5], fo[5];
           face_frame(L, d, ql);
           face_frame(R, d, qr);
-          hllc_f32(ql, qr, c, smallc2, dtdx, ff);
+          riemann_f32<RS>(ql, qr, c, smallc2, dtdx, ff);
           flux_back(ff, d, fo);
           (yf ? fy4 : fx4)[fsl] = make_float4(fo[0], fo[1], fo[2], fo[3]);
           (yf ? fy1 : fx1)[fsl] = fo[4];
@@ -354,14 +354,14 @@ __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int
 
 // One step of one problem: one CTA per work item. MINB: CTAs per SM the
 // register allocation is bounded for.
-template <int TX, int TY, int MINB, int ST>
+template <int TX, int TY, int MINB, int RS, int ST>
 __global__ void __launch_bounds__(S2Geom<TX, TY>::NT, MINB) stream2_step_kernel(StreamArgs a) {
-  stream2_step_body<TX, TY, ST>(a, blockIdx.x);
+  stream2_step_body<TX, TY, RS, ST>(a, blockIdx.x);
 }
 
 // One round of the serving engine over the work items of every active
 // problem (the BatchDesc protocol of stream_batch_kernel).
-template <int TX, int TY, int MINB, int ST>
+template <int TX, int TY, int MINB, int RS, int ST>
 __global__ void __launch_bounds__(S2Geom<TX, TY>::NT, MINB)
     stream2_batch_kernel(const BatchDesc* __restrict__ desc, const int32_t* __restrict__ item_off, int nprob) {
   const int b = blockIdx.x;
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(S2Geom<TX, TY>::NT, MINB)
   a.uin = d.dense[cur];
   a.uout = d.dense[cur ^ 1];
   a.dt_dev = d.clock;
-  stream2_step_body<TX, TY, ST>(a, b - item_off[lo]);
+  stream2_step_body<TX, TY, RS, ST>(a, b - item_off[lo]);
 }
 
 }  // namespace rb

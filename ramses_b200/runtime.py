@@ -25,7 +25,7 @@ RB_PREC_MIXED = 1
 MAXLEVEL = 32
 # z-streaming column shapes (TX, TY, CTAs per SM of register budget), as
 # kStreamShapes in csrc/tile_launch.h; STREAM2_SHAPES run stream2_step_kernel
-# (FP32-mixed, HLLC with minmod or moncen slopes)
+# (FP32-mixed; llf, hll or hllc with minmod or moncen slopes)
 STREAM_SHAPES = [(8, 8, 1), (16, 8, 1), (16, 16, 1), (16, 8, 2), (8, 8, 4), (16, 8, 3), (16, 8, 2)]
 STREAM2_SHAPES = (5, 6)
 
