@@ -2421,7 +2421,7 @@ static int uniform_run_dense(rb_context* c, int nsteps, int use_graph, double* t
     c->dense_valid = true;
     drop_graph(c);
   }
-  RB_TRY(ensure_partial(c, std::max<int64_t>(c->stream_items, grid_for((int64_t)L.noct * 8, 256, 148 * 8))));
+  RB_TRY(ensure_partial(c, grid_for((int64_t)L.noct * 8, 256, 148 * 8)));
   if (!c->clock_valid) {
     const int nblk = grid_for((int64_t)L.noct * 8, 256, 148 * 8);
     rb::courant_partial_kernel<256><<<nblk, 256, 0, c->stream>>>(c->d_uold, c->d_son, L.d_active, L.noct, c->ncell,
@@ -2440,7 +2440,13 @@ static int uniform_run_dense(rb_context* c, int nsteps, int use_graph, double* t
   }
   rb::StreamArgs sa;
   memset(&sa, 0, sizeof sa);
-  sa.partial = c->d_partial;
+  sa.clk.clock = c->d_clock;
+  sa.clk.smax = c->d_cfl;
+  sa.clk.count = (unsigned*)(c->d_cfl + 1);
+  sa.clk.nitems = c->stream_items;
+  sa.clk.dt_max = dt_max;
+  sa.clk.dt0 = dt0;
+  sa.clk.t_end = sa.clk.max_steps = HUGE_VAL;
   sa.dt_dev = c->d_clock;
   sa.nx = c->dnx; sa.ny = c->dny; sa.nz = c->dnz;
   sa.hz = c->stream_hz;
@@ -2458,9 +2464,6 @@ static int uniform_run_dense(rb_context* c, int nsteps, int use_graph, double* t
                         : rb::launch_stream_f64(c->stream_shape, sa, c->stream_items, c->stream);
     if (e != cudaSuccess) return fail(RB_ERR_CUDA, "stream kernel launch failed: %s", cudaGetErrorString(e));
     if (timed) RB_CUDA(cudaEventRecord(c->evpool[2 * s_idx + 1], c->stream));
-    rb::reduce_partials_kernel<<<1, RB_RED_NT, 0, c->stream>>>(c->d_partial, c->stream_items, dt_max, dt0, 1,
-                                                              c->d_clock, 1);
-    RB_CUDA(cudaGetLastError());
     return RB_OK;
   };
   if (nsteps > 0) {
@@ -2564,12 +2567,10 @@ int rb_autotune_uniform(rb_context* c, int* shape_out, int* hz_out, float* ms_ou
       if (c->dnz % hz != 0) continue;
       const int items = stream_items_of(c, s, hz);
       if (items < 148 && hz != 4) continue;
-      RB_TRY(ensure_partial(c, items));
       rb::StreamArgs sa;
       memset(&sa, 0, sizeof sa);
       sa.uin = c->d_dense[c->dense_cur];
       sa.uout = c->d_dense[c->dense_cur ^ 1];
-      sa.partial = c->d_partial;
       sa.dt_dev = c->d_red + 4;
       sa.nx = c->dnx; sa.ny = c->dny; sa.nz = c->dnz;
       sa.hz = hz;

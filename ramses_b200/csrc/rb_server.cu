@@ -6,7 +6,7 @@
 //  * dense: one complete level as a periodic Cartesian grid (the layout of the
 //    z-streaming kernel). All active dense problems advance together: every
 //    step is ONE launch of stream_batch_kernel over the work items of all of
-//    them, then one batch_clock_kernel launch that advances each problem's own
+//    them, in which the last CTA of each problem advances the problem's own
 //    clock. Problems never share a reduction or an atomic, so a problem's
 //    result does not depend on which others share its launches.
 //  * octree: an AMR problem with its own rb_context, stepped by device-
@@ -85,13 +85,13 @@ struct rb_server {
   // device clocks of the dense problems: [kMaxSlots][8], read back whole
   double* d_clocks = nullptr;
   double* h_clocks[2] = {nullptr, nullptr};
-  unsigned long long* d_smax = nullptr;  // [kMaxSlots] scratch of the first dt
+  unsigned long long* d_smax = nullptr;  // [kMaxSlots] largest wave speed of the step under way
+  unsigned* d_count = nullptr;           // [kMaxSlots] CTAs done of the step under way
   std::vector<int> free_slots;
   // round buffers
   rb::BatchDesc* d_desc = nullptr;
   int32_t* d_off = nullptr;
-  double* d_partial = nullptr;
-  int desc_cap = 0, item_cap = 0;
+  int desc_cap = 0;
   rb::BatchDesc* h_desc[2] = {nullptr, nullptr};
   int32_t* h_off[2] = {nullptr, nullptr};
   int hcap[2] = {0, 0};
@@ -125,7 +125,7 @@ int pick_hz(int nx, int ny, int nz, int tx, int ty) {
   return hz;
 }
 
-int grow_round_buffers(rb_server* s, int nprob, int nitems) {
+int grow_round_buffers(rb_server* s, int nprob) {
   if (nprob + 1 > s->desc_cap) {
     int cap = std::max(nprob + 1, 2 * s->desc_cap);
     if (s->d_desc) cudaFreeAsync(s->d_desc, s->stream);
@@ -133,12 +133,6 @@ int grow_round_buffers(rb_server* s, int nprob, int nitems) {
     RB_CUDA(cudaMallocAsync((void**)&s->d_desc, cap * sizeof(rb::BatchDesc), s->stream));
     RB_CUDA(cudaMallocAsync((void**)&s->d_off, (cap + 1) * sizeof(int32_t), s->stream));
     s->desc_cap = cap;
-  }
-  if (nitems > s->item_cap) {
-    int cap = std::max(nitems, 2 * s->item_cap);
-    if (s->d_partial) cudaFreeAsync(s->d_partial, s->stream);
-    RB_CUDA(cudaMallocAsync((void**)&s->d_partial, (size_t)cap * 4 * sizeof(double), s->stream));
-    s->item_cap = cap;
   }
   const int k = s->round & 1;
   if (nprob + 1 > s->hcap[k]) {
@@ -257,7 +251,7 @@ int launch_round(rb_server* s) {
   for (Request* r : s->dense) nitems += r->items;
   const int nprob = (int)s->dense.size();
   if (nprob) {
-    RB_TRY(grow_round_buffers(s, nprob, nitems));
+    RB_TRY(grow_round_buffers(s, nprob));
     rb::BatchDesc* hd = s->h_desc[k];
     int32_t* ho = s->h_off[k];
     int off = 0;
@@ -265,7 +259,14 @@ int launch_round(rb_server* s) {
       Request* r = s->dense[p];
       rb::BatchDesc& d = hd[p];
       memset(&d, 0, sizeof d);
-      d.a.partial = s->d_partial + (int64_t)off * 4;
+      d.a.clk.clock = s->d_clocks + (int64_t)r->slot * 8;
+      d.a.clk.smax = s->d_smax + r->slot;
+      d.a.clk.count = s->d_count + r->slot;
+      d.a.clk.nitems = r->items;
+      d.a.clk.dt_max = r->dx * r->nx / s->hp.smallc;
+      d.a.clk.dt0 = s->hp.courant_factor * r->dx / s->hp.smallc;
+      d.a.clk.t_end = r->t_end;
+      d.a.clk.max_steps = (double)r->max_steps;
       d.a.nx = r->nx; d.a.ny = r->ny; d.a.nz = r->nz;
       d.a.hz = r->hz;
       d.a.outflow = r->outflow;
@@ -277,13 +278,7 @@ int launch_round(rb_server* s) {
       const int64_t n = (int64_t)r->nx * r->ny * r->nz;
       d.dense[0] = r->d_buf;
       d.dense[1] = r->d_buf + 5 * n;
-      d.clock = s->d_clocks + (int64_t)r->slot * 8;
-      d.t_end = r->t_end;
-      d.max_steps = (double)r->max_steps;
-      d.dt_max = r->dx * r->nx / s->hp.smallc;
-      d.dt0 = s->hp.courant_factor * r->dx / s->hp.smallc;
       d.parity0 = 0;
-      d.nitems = r->items;
       ho[p] = off;
       off += r->items;
       s->round_members[k].push_back(r);
@@ -296,8 +291,6 @@ int launch_round(rb_server* s) {
                           ? rb::launch_batch_mixed(s->shape, s->hp, s->d_desc, s->d_off, nprob, nitems, s->stream)
                           : rb::launch_batch_f64(s->shape, s->hp, s->d_desc, s->d_off, nprob, nitems, s->stream);
       if (e != cudaSuccess) return fail(RB_ERR_CUDA, "batched step launch failed: %s", cudaGetErrorString(e));
-      rb::batch_clock_kernel<<<nprob, RB_RED_NT, 0, s->stream>>>(s->d_desc, s->d_off);
-      RB_CUDA(cudaGetLastError());
       s->batch_launches++;
     }
     int maxslot = 0;
@@ -451,12 +444,14 @@ int rb_server_create(const rb_hydro_params* hp, int precision, int64_t hbm_budge
       cudaEventCreateWithFlags(&s->round_ev[1], cudaEventDisableTiming) != cudaSuccess)
     return bail(fail(RB_ERR_CUDA, "stream/event creation failed"));
   int rc;
-  if ((rc = dalloc(&s->d_clocks, (size_t)kMaxSlots * 8)) || (rc = dalloc(&s->d_smax, (size_t)kMaxSlots)))
+  if ((rc = dalloc(&s->d_clocks, (size_t)kMaxSlots * 8)) || (rc = dalloc(&s->d_smax, (size_t)kMaxSlots)) ||
+      (rc = dalloc(&s->d_count, (size_t)kMaxSlots)))
     return bail(rc);
   if (cudaMallocHost((void**)&s->h_clocks[0], (size_t)kMaxSlots * 8 * sizeof(double)) != cudaSuccess ||
       cudaMallocHost((void**)&s->h_clocks[1], (size_t)kMaxSlots * 8 * sizeof(double)) != cudaSuccess)
     return bail(fail(RB_ERR_NOMEM, "pinned allocation failed"));
   if (cudaMemsetAsync(s->d_clocks, 0, (size_t)kMaxSlots * 8 * sizeof(double), s->stream) != cudaSuccess ||
+      cudaMemsetAsync(s->d_count, 0, (size_t)kMaxSlots * sizeof(unsigned), s->stream) != cudaSuccess ||
       cudaStreamSynchronize(s->stream) != cudaSuccess)
     return bail(fail(RB_ERR_CUDA, "initialising the clock pool failed"));
   s->free_slots.reserve(kMaxSlots);
@@ -480,10 +475,10 @@ int rb_server_destroy(rb_server* s) {
   for (Request* r : s->dense) release_dense(s, r);
   if (s->d_desc) cudaFreeAsync(s->d_desc, s->stream);
   if (s->d_off) cudaFreeAsync(s->d_off, s->stream);
-  if (s->d_partial) cudaFreeAsync(s->d_partial, s->stream);
   if (s->stream) cudaStreamSynchronize(s->stream);
   dfree(s->d_clocks);
   dfree(s->d_smax);
+  dfree(s->d_count);
   for (int k = 0; k < 2; k++) {
     if (s->h_clocks[k]) cudaFreeHost(s->h_clocks[k]);
     if (s->h_desc[k]) cudaFreeHost(s->h_desc[k]);

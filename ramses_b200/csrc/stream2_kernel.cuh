@@ -65,6 +65,86 @@ struct S2Geom {
   static_assert(RAW_BYTES % 16 == 0 && Q4_BYTES % 16 == 0 && QP_BYTES % 16 == 0, "16-byte aligned sections");
 };
 
+// This kernel's own forms of hllc_f32, half_step and face_pair
+// (hydro_core.cuh), with the contraction left to the compiler: one reciprocal
+// per face for the two sound speeds instead of two, and the rounding that
+// long runs of this kernel have been compared at (a strong shock tube
+// amplifies another rounding to 1e-4 in 200 steps). Density products stay
+// above 1e-38 for densities above 1e-19.
+// HLLC flux (riemann_hllc, godunov_utils.f90:988-1209) in FP32 for the mixed
+// path, times dt/dx. Face frame (rho, u_n, P, u_t1, u_t2) in, flux of (mass,
+// normal momentum, energy, t1 momentum, t2 momentum) out. The larger of the
+// two fast sound speeds is formed with one reciprocal and one square root,
+// and the sampled state's side is chosen before its energy is formed.
+__device__ __forceinline__ void hllc_stream(const float ql[5], const float qr[5], const Consts<float>& c,
+                                         float smallc2, float dtdx, float f[5]) {
+  const float rl = fmaxf(ql[0], c.smallr), ul = ql[1], Pl = fmaxf(ql[2], rl * c.smallp);
+  const float rr = fmaxf(qr[0], c.smallr), ur = qr[1], Pr = fmaxf(qr[2], rr * c.smallp);
+  // max(gamma Pl/rl, gamma Pr/rr, smallc^2), rl, rr > 0
+  const float a2 = fmaxf(fmaxf(Pl * rr, Pr * rl) * (c.gamma * __fdividef(1.0f, rl * rr)), smallc2);
+  const float cmax = sqrtf(a2);
+  const float SL = fminf(ul, ur) - cmax, SR = fmaxf(ul, ur) + cmax;
+  const float rcl = rl * (ul - SL), rcr = rr * (SR - ur);
+  const float inv = __fdividef(1.0f, rcr + rcl);
+  const float ustar = (rcr * ur + rcl * ul + (Pl - Pr)) * inv;
+  const float Pstar = (rcr * Pl + rcl * Pr + rcl * rcr * (ul - ur)) * inv;
+  // sampling at x/t = 0: outer left if SL > 0, left star if ustar > 0, right
+  // star if SR > 0, else outer right
+  const bool outl = SL > 0.0f, lft = ustar > 0.0f;
+  const bool side = outl || lft;
+  const bool star = !outl && (lft || SR > 0.0f);
+  const float rs = side ? rl : rr, us = side ? ul : ur, Ss = side ? SL : SR, Ps = side ? Pl : Pr;
+  const float t1 = side ? ql[3] : qr[3], t2 = side ? ql[4] : qr[4];
+  const float num = Ss - us, iden = __fdividef(1.0f, Ss - ustar);
+  const float ratio = star ? num * iden : 1.0f;
+  const float ro = rs * ratio;
+  const float uo = star ? ustar : us;
+  const float Po = star ? Pstar : Ps;
+  const float ets = Ps * c.entho + 0.5f * rs * (us * us + t1 * t1 + t2 * t2);
+  const float eto = star ? (num * ets - Ps * us + Pstar * ustar) * iden : ets;
+  const float uos = uo * dtdx;
+  const float mo = ro * uos;
+  f[0] = mo;
+  f[1] = mo * uo + Po * dtdx;
+  f[2] = (eto + Po) * uos;
+  f[3] = mo * t1;
+  f[4] = mo * t2;
+}
+
+// MUSCL-Hancock half-step state of a cell for the FP32 path: h = q + s dt/(2dx)
+// with the source terms of trace3d (umuscl.f90:576-580), equal in every
+// direction on a cubic cell. hd[v][d] are half slopes; th = dt/dx (the factor
+// 1/2 of the half step cancels the 2 of the full slope).
+__device__ __forceinline__ void half_step_stream(const Prim<float>& q, const float hd[5][3], float gamma, float th,
+                                          float h[5]) {
+  const float r = q.r, u = q.u, v = q.v, w = q.w, p = q.p;
+  const float divv = hd[1][0] + hd[2][1] + hd[3][2];
+  const float ir = __fdividef(1.0f, r);
+  h[0] = r - th * (u * hd[0][0] + v * hd[0][1] + w * hd[0][2] + divv * r);
+  h[4] = p - th * (u * hd[4][0] + v * hd[4][1] + w * hd[4][2] + divv * (gamma * p));
+  h[1] = u - th * (u * hd[1][0] + v * hd[1][1] + w * hd[1][2] + hd[4][0] * ir);
+  h[2] = v - th * (u * hd[2][0] + v * hd[2][1] + w * hd[2][2] + hd[4][1] * ir);
+  h[3] = w - th * (u * hd[3][0] + v * hd[3][1] + w * hd[3][2] + hd[4][2] * ir);
+}
+
+// face states of direction d: right state at the lower face P = h - hd,
+// left state at the upper face M = h + hd, density floored to the cell's
+// (trace3d: if (q < smallr) q = r)
+__device__ __forceinline__ void face_pair_stream(const float h[5], const float hd[5][3], int d, float r, float smallr,
+                                          float P[5], float M[5]) {
+#pragma unroll
+  for (int v = 0; v < 5; v++) { P[v] = h[v] - hd[v][d]; M[v] = h[v] + hd[v][d]; }
+  if (P[0] < smallr) P[0] = r;
+  if (M[0] < smallr) M[0] = r;
+}
+
+template <int RS>
+__device__ __forceinline__ void riemann_stream(const float ql[5], const float qr[5], const Consts<float>& c,
+                                               float smallc2, float dtdx, float f[5]) {
+  if constexpr (RS == RB_RIEMANN_HLLC) hllc_stream(ql, qr, c, smallc2, dtdx, f);
+  else llf_hll_f32<RS, false>(ql, qr, c, dtdx, f);
+}
+
 // One work item (TX x TY column, z range [z0, z0+hz)) of one problem.
 template <int TX, int TY, int RS, int ST>
 __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int item) {
@@ -222,17 +302,17 @@ __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int
         dzl[v] = bz[v];
       }
       float h[5];
-      half_step(q_0, hd, c.gamma, th, h);
+      half_step_stream(q_0, hd, c.gamma, th, h);
       float P[5], M[5];
-      face_pair(h, hd, 0, q_0.r, c.smallr, P, M);
+      face_pair_stream(h, hd, 0, q_0.r, c.smallr, P, M);
       fs[slot] = make_float4(M[0], M[1], M[2], M[3]);
       fs[G::NC + slot] = make_float4(P[0], P[1], P[2], P[3]);
       const float mxp = M[4], pxp_ = P[4];
-      face_pair(h, hd, 1, q_0.r, c.smallr, P, M);
+      face_pair_stream(h, hd, 1, q_0.r, c.smallr, P, M);
       fs[2 * G::NC + slot] = make_float4(M[0], M[1], M[2], M[3]);
       fs[3 * G::NC + slot] = make_float4(P[0], P[1], P[2], P[3]);
       fs[4 * G::NC + slot] = make_float4(mxp, pxp_, M[4], P[4]);
-      if (inner) face_pair(h, hd, 2, q_0.r, c.smallr, zP, zM);
+      if (inner) face_pair_stream(h, hd, 2, q_0.r, c.smallr, zP, zM);
     }
     cp_async_wait<0>();                    // raw plane k+2 (own copies) has landed
     __syncthreads();                       // B1: face states and raw plane k+2 visible
@@ -255,7 +335,7 @@ __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int
         float ql[5], qr[5], ff[5], fo[5];
         face_frame(L, 0, ql);
         face_frame(R, 0, qr);
-        riemann_f32<RS>(ql, qr, c, smallc2, dtdx, ff);
+        riemann_stream<RS>(ql, qr, c, smallc2, dtdx, ff);
         flux_back(ff, 0, fo);
         fx4[slot] = make_float4(fo[0], fo[1], fo[2], fo[3]);
         fx1[slot] = fo[4];
@@ -264,7 +344,7 @@ __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int
         float ql[5], qr[5], ff[5], fo[5];
         face_frame(qmz, 2, ql);
         face_frame(zP, 2, qr);
-        riemann_f32<RS>(ql, qr, c, smallc2, dtdx, ff);
+        riemann_stream<RS>(ql, qr, c, smallc2, dtdx, ff);
         flux_back(ff, 2, fo);
 #pragma unroll
         for (int v = 0; v < 5; v++) fzd[v] = (double)fo[v];
@@ -290,7 +370,7 @@ __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int
           float ql[5], qr[5], ff[5], fo[5];
           face_frame(L, d, ql);
           face_frame(R, d, qr);
-          riemann_f32<RS>(ql, qr, c, smallc2, dtdx, ff);
+          riemann_stream<RS>(ql, qr, c, smallc2, dtdx, ff);
           flux_back(ff, d, fo);
           (yf ? fy4 : fx4)[fsl] = make_float4(fo[0], fo[1], fo[2], fo[3]);
           (yf ? fy1 : fx1)[fsl] = fo[4];
@@ -338,17 +418,14 @@ __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int
   }
   cp_async_wait<0>();
 
-  // ---- CFL partial of this work item (max wave speed -> min dt) ----
+  // ---- the work item's largest wave speed, and the clock ----
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) smax = fmax(smax, __shfl_xor_sync(0xffffffffu, smax, o));
   if ((tid & 31) == 0) red[tid >> 5] = smax;
   __syncthreads();
   if (tid == 0) {
     for (int w = 1; w < G::NT / 32; w++) smax = fmax(smax, red[w]);
-    a.partial[(int64_t)item * 4 + 0] = smax > 0.0 ? cfl_dt_from_speed(smax, a.dx, a.hp.courant_factor) : 1.0e300;
-    a.partial[(int64_t)item * 4 + 1] = 0.0;
-    a.partial[(int64_t)item * 4 + 2] = 0.0;
-    a.partial[(int64_t)item * 4 + 3] = 0.0;
+    stream_clock(a.clk, smax, a.dx, a.hp.courant_factor);
   }
 }
 
@@ -371,12 +448,12 @@ __global__ void __launch_bounds__(S2Geom<TX, TY>::NT, MINB)
     if (item_off[mid] <= b) lo = mid; else hi = mid - 1;
   }
   const BatchDesc& d = desc[lo];
-  if (d.clock[6] != 0.0) return;  // finished: the state stays where it is
+  if (d.a.clk.clock[6] != 0.0) return;  // finished: the state stays where it is
   StreamArgs a = d.a;
-  const int cur = (d.parity0 + (int)d.clock[5]) & 1;
+  const int cur = (d.parity0 + (int)d.a.clk.clock[5]) & 1;
   a.uin = d.dense[cur];
   a.uout = d.dense[cur ^ 1];
-  a.dt_dev = d.clock;
+  a.dt_dev = d.a.clk.clock;
   stream2_step_body<TX, TY, RS, ST>(a, b - item_off[lo]);
 }
 
