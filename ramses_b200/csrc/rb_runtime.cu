@@ -1211,13 +1211,29 @@ bool stream_shape_fits(const rb_context* c, int s) {
 int stream_items_of(const rb_context* c, int s, int hz) {
   return (c->dnx / rb::kStreamShapes[s][0]) * (c->dny / rb::kStreamShapes[s][1]) * (c->dnz / hz);
 }
-// z extent of a work item: the longest power of two <= 64 dividing nz that
-// still gives >= 4 work items per SM
-int default_stream_hz(const rb_context* c, int s) {
-  int hz = 64;
-  while (hz > 2 && (c->dnz % hz != 0 || stream_items_of(c, s, hz) < 4 * 148)) hz >>= 1;
-  if (c->dnz % hz != 0) hz = 2;
-  return hz;
+// Default z-streaming configuration. A work item of hz planes streams hz + 2
+// and has a prologue of about two more, and the items run in waves of the CTAs
+// that fit at once, so the time follows ceil(items / slots) * (hz + 4) planes.
+// Measured per step (us) and in those units, FP32-mixed 16x8 columns at 2 CTAs
+// per SM: 64^3 hz 2/4/8/16: 44/33/27/35, 24/16/12/20; 128^3 hz 8/16/32/64:
+// 150/135/133/128, 84/80/72/68; 256^3 hz 16/32/64: 945/873/837, 560/504/476.
+// FP64 16x16 columns: 64^3 hz 2/4/8/16: 99/78/67/115, 24/16/12/20. A plane of
+// a narrower column is cheaper when the CTAs do not fill the GPU (32^3 FP64:
+// 29 us with 64 CTAs of 16x16, 24.5 with 128 of 16x8; 16^3: 22.6 with 8x8).
+void default_stream_config(const rb_context* c, int* shape, int* hz) {
+  *shape = -1;
+  double best = HUGE_VAL;
+  struct { int s; double plane; } cand[] = {{6, 1.0}, {2, 1.0}, {1, 0.83}, {0, 0.78}};
+  for (const auto& k : cand) {
+    if (!stream_shape_fits(c, k.s)) continue;
+    const int slots = 148 * rb::kStreamShapes[k.s][2];
+    for (int h = 64; h >= 2; h >>= 1) {
+      if (c->dnz % h != 0) continue;
+      const double t = k.plane * ((stream_items_of(c, k.s, h) + slots - 1) / slots) * (h + 4);
+      if (t < best) { best = t; *shape = k.s; *hz = h; }
+    }
+    if (k.s == 6) return;  // where it fits, the balanced kernel is the fastest
+  }
 }
 
 // Allocate the dense mirror of the finest level (complete by construction of
@@ -1239,16 +1255,8 @@ int dense_prepare(rb_context* c) {
   }
   RB_TRY(dalloc(&c->d_cbase, cb.size()));
   RB_TRY(h2d(c, c->d_cbase, cb.data(), cb.size() * 8));
-  // default column shape: the FP32-mixed kernel of stream2_kernel.cuh where
-  // it applies, else the widest of 16x16, 16x8, 8x8 that divides the grid
-  int shape = -1;
-  for (int s : {6, 2, 1, 0})
-    if (stream_shape_fits(c, s)) { shape = s; break; }
-  c->stream_shape = shape;
-  if (shape >= 0) {
-    c->stream_hz = default_stream_hz(c, shape);
-    c->stream_items = stream_items_of(c, shape, c->stream_hz);
-  }
+  default_stream_config(c, &c->stream_shape, &c->stream_hz);
+  if (c->stream_shape >= 0) c->stream_items = stream_items_of(c, c->stream_shape, c->stream_hz);
   c->dense_valid = false;
   return RB_OK;
 }
