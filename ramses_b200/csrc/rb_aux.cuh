@@ -4,9 +4,11 @@
 // the Fortran arrays and the device layout.
 //
 // Device layout: variable-major, then oct-major: u[v*ncell + dc] with
-// dc = icell-1 for the ncoarse coarse cells and dc = ncoarse + 8*(igrid-1) +
-// (ind-1) for child slot ind of oct igrid, so an oct's 8 cells of one
-// variable are one 64-byte row.
+// dc = icell-1 for the coarse cells and dc = oct0 + 8*(igrid-1) + (ind-1) for
+// child slot ind of oct igrid. oct0 (the kernels' argument ncoarse, ncell the
+// stride of the variables) and the stride are multiples of 8, so an oct's 8
+// cells of one variable are one aligned 64-byte row: two 32-byte sectors, where
+// rows that start at ncoarse = 1 touched three.
 #pragma once
 #include <cstdint>
 
@@ -20,12 +22,12 @@ namespace rb {
     if ((g) != nullptr && *(g) != 0.0) return;    \
   } while (0)
 
-__device__ __forceinline__ int64_t dev_cell_of_fortran(int64_t icell /*1-based*/, int32_t ncoarse,
+__device__ __forceinline__ int64_t dev_cell_of_fortran(int64_t icell /*1-based*/, int32_t ncoarse, int32_t oct0,
                                                        int32_t ngridmax) {
   if (icell <= ncoarse) return icell - 1;
   const int64_t r = icell - 1 - ncoarse;
   const int64_t ind = r / ngridmax, ig = r % ngridmax;  // ig = igrid-1
-  return ncoarse + ig * 8 + ind;
+  return oct0 + ig * 8 + ind;
 }
 
 // Fortran uold(ncell,5) -> device layout. The coarse cells keep their index;
@@ -35,13 +37,14 @@ __device__ __forceinline__ int64_t dev_cell_of_fortran(int64_t icell /*1-based*/
 // and reads one 32-byte sector in each of the 8 Fortran rows; the nvar values
 // of a cell are in flight together.
 static __global__ void permute_f2d_kernel(const double* __restrict__ f, double* __restrict__ d, int64_t ncell,
-                                          int32_t ncoarse, int32_t ngridmax, int nvar) {
+                                 int64_t dcell, int32_t ncoarse, int32_t oct0, int32_t ngridmax, int nvar) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ncell; i += stride) {
-    int64_t fi = i;
+    int64_t fi = i, di = i;
     if (i >= ncoarse) {
       const int64_t r = i - ncoarse;
       fi = ncoarse + (r & 7) * (int64_t)ngridmax + (r >> 3);
+      di = oct0 + r;
     }
     double x[5];
 #pragma unroll
@@ -49,18 +52,18 @@ static __global__ void permute_f2d_kernel(const double* __restrict__ f, double* 
       if (v < nvar) x[v] = f[v * ncell + fi];
 #pragma unroll
     for (int v = 0; v < 5; v++)
-      if (v < nvar) d[v * ncell + i] = x[v];
+      if (v < nvar) d[v * dcell + di] = x[v];
   }
 }
 // Device layout -> Fortran: Fortran order (whole Fortran rows written), one
 // value per iteration; the device reads of a warp hit 32 octs' cells of one
 // child, and the other children's warps find those sectors in L2.
 static __global__ void permute_d2f_kernel(const double* __restrict__ d, double* __restrict__ f, int64_t ncell,
-                                          int32_t ncoarse, int32_t ngridmax, int nvar) {
+                                   int64_t dcell, int32_t ncoarse, int32_t oct0, int32_t ngridmax, int nvar) {
   const int64_t n = ncell * nvar;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t v = i / ncell, icell = i % ncell + 1;
-    f[i] = d[v * ncell + dev_cell_of_fortran(icell, ncoarse, ngridmax)];
+    f[i] = d[v * dcell + dev_cell_of_fortran(icell, ncoarse, oct0, ngridmax)];
   }
 }
 // The cells of one level's octs between the staging copy of uold in the
@@ -70,16 +73,16 @@ static __global__ void permute_d2f_kernel(const double* __restrict__ d, double* 
 template <bool F2D>
 static __global__ void permute_level_kernel(double* __restrict__ f, double* __restrict__ d,
                                             const int32_t* __restrict__ act, int64_t noct, int64_t ncell,
-                                            int32_t ncoarse, int32_t ngridmax) {
+                                            int64_t dcell, int32_t ncoarse, int32_t oct0, int32_t ngridmax) {
   const int64_t n = noct * 8;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t g = act[i >> 3];
     const int ind = (int)(i & 7);
-    const int64_t fi = ncoarse + (int64_t)ind * ngridmax + g, di = ncoarse + 8 * g + ind;
+    const int64_t fi = ncoarse + (int64_t)ind * ngridmax + g, di = oct0 + 8 * g + ind;
 #pragma unroll
     for (int v = 0; v < 5; v++) {
-      if (F2D) d[v * ncell + di] = f[v * ncell + fi];
-      else f[v * ncell + fi] = d[v * ncell + di];
+      if (F2D) d[v * dcell + di] = f[v * ncell + fi];
+      else f[v * ncell + fi] = d[v * dcell + di];
     }
   }
 }
@@ -91,9 +94,9 @@ static __global__ void scatter_son_kernel(int32_t* __restrict__ d, const int64_t
 }
 
 static __global__ void permute_son_kernel(const int32_t* __restrict__ f, int32_t* __restrict__ d, int64_t ncell,
-                                   int32_t ncoarse, int32_t ngridmax) {
+                                   int32_t ncoarse, int32_t oct0, int32_t ngridmax) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ncell; i += (int64_t)gridDim.x * blockDim.x)
-    d[dev_cell_of_fortran(i + 1, ncoarse, ngridmax)] = f[i];
+    d[dev_cell_of_fortran(i + 1, ncoarse, oct0, ngridmax)] = f[i];
 }
 
 // Internal energy E - d/2 (u^2+v^2+w^2), d = max(rho, smallr), u = m/d, of
@@ -595,7 +598,8 @@ __device__ __forceinline__ void cfl_tail(double smax, const CflTail& t) {
 // The CFL condition of level l's leaf cells in state u: before a run's first
 // step (with unew non-null also set_unew, unew = u), and after each step of a
 // finest level, whose state needs no set_uold pass (see amr_step_dev).
-// FAST (FP32-mixed contexts): the wave speed of cfl_speed_fast.
+// son null: a level without split cells. FAST (FP32-mixed contexts): the wave
+// speed of cfl_speed_fast.
 template <int NT, bool FAST>
 static __global__ void __launch_bounds__(NT) level_cfl_kernel(const double* __restrict__ u,
                                                               const int32_t* __restrict__ son,
@@ -606,19 +610,29 @@ static __global__ void __launch_bounds__(NT) level_cfl_kernel(const double* __re
                                                               const __grid_constant__ CflTail tail) {
   RB_GATE(gate);
   double smax = 0.0;
-  const int64_t n = (int64_t)noct * 8;
-  for (int64_t i = blockIdx.x * (int64_t)NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT) {
-    const int64_t dc = ncoarse + (int64_t)active[i >> 3] * 8 + (i & 7);
-    const bool leaf = son[dc] == 0;
-    if (!leaf && !unew) continue;
-    double q[5];
+  const int64_t n = (int64_t)noct * 8, st = (int64_t)gridDim.x * NT;
+  // two cells in flight per thread
+  for (int64_t i = blockIdx.x * (int64_t)NT + threadIdx.x; i < n; i += 2 * st) {
+    double q[2][5];
+    bool leaf[2];
 #pragma unroll
-    for (int v = 0; v < 5; v++) q[v] = u[v * ncell + dc];
-    if (unew) {
+    for (int k = 0; k < 2; k++) {
+      const int64_t j = i + k * st;
+      leaf[k] = false;
+      if (j >= n) continue;
+      const int64_t dc = ncoarse + (int64_t)active[j >> 3] * 8 + (j & 7);
+      leaf[k] = son == nullptr || son[dc] == 0;
+      if (!leaf[k] && !unew) continue;
 #pragma unroll
-      for (int v = 0; v < 5; v++) unew[v * ncell + dc] = q[v];
+      for (int v = 0; v < 5; v++) q[k][v] = u[v * ncell + dc];
+      if (unew) {
+#pragma unroll
+        for (int v = 0; v < 5; v++) unew[v * ncell + dc] = q[k][v];
+      }
     }
-    if (leaf) smax = fmx(smax, FAST ? cfl_speed_fast(q, hp) : cfl_speed(q, hp));
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+      if (leaf[k]) smax = fmx(smax, FAST ? cfl_speed_fast(q[k], hp) : cfl_speed(q[k], hp));
   }
   cfl_tail<NT>(smax, tail);
 }
@@ -720,20 +734,32 @@ static __global__ void hydro_flag_kernel(const double* __restrict__ uold, const 
 // upload_fine / upl (interpol_hydro.f90:5-263): restriction of every split
 // cell of the level's active octs from its 8 children.
 // Restriction of one split cell dc from its 8 children (oct gs).
-__device__ __forceinline__ void restrict_cell(double* __restrict__ uold, int64_t dc, int gs, int64_t ncell,
-                                              int32_t ncoarse, const rb_hydro_params& hp) {
+// next, if non-null, gets the same values.
+__device__ __forceinline__ void restrict_cell(double* uold, int64_t dc, int gs, int64_t ncell, int32_t ncoarse,
+                                              const rb_hydro_params& hp, double* next) {
   {
     const int64_t c0 = ncoarse + (int64_t)(gs - 1) * 8;
-    double getx = 0.0;
-    for (int is = 0; is < 8; is++) getx = getx + fmx(uold[c0 + is], hp.smallr);
-    uold[dc] = getx / 8.0;
-    for (int v = 1; v < 5; v++) {
-      getx = 0.0;
-      for (int is = 0; is < 8; is++) getx = getx + uold[v * ncell + c0 + is];
-      uold[v * ncell + dc] = getx / 8.0;
+    // one variable at a time, its children's row in four 16-byte loads: more
+    // rows at once cost the pass more occupancy than they give it (all five:
+    // 22.1 against 18.6 us on levels 5-8)
+#pragma unroll 1
+    for (int v = 0; v < 5; v++) {
+      const double2* row = reinterpret_cast<const double2*>(uold + v * ncell + c0);
+      double2 ch[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) ch[k] = row[k];
+      double getx = 0.0;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        getx = getx + (v == 0 ? fmx(ch[k].x, hp.smallr) : ch[k].x);
+        getx = getx + (v == 0 ? fmx(ch[k].y, hp.smallr) : ch[k].y);
+      }
+      getx = getx / 8.0;
+      uold[v * ncell + dc] = getx;
+      if (next != nullptr) next[v * ncell + dc] = getx;
     }
     if (hp.interpol_var == 1 || hp.interpol_var == 2) {
-      getx = 0.0;
+      double getx = 0.0;
       for (int is = 0; is < 8; is++) {
         const int64_t sc = c0 + is;
         double ekin = 0.0;
@@ -746,7 +772,9 @@ __device__ __forceinline__ void restrict_cell(double* __restrict__ uold, int64_t
       for (int d = 1; d <= 3; d++)
         ekin = ekin + 0.5 * (uold[d * ncell + dc] * uold[d * ncell + dc]) / fmx(uold[dc], hp.smallr);
       const double erad = 0.0;
-      uold[4 * ncell + dc] = getx / 8.0 + ekin + erad;
+      const double e = getx / 8.0 + ekin + erad;
+      uold[4 * ncell + dc] = e;
+      if (next != nullptr) next[4 * ncell + dc] = e;
     }
   }
 }
@@ -759,7 +787,7 @@ static __global__ void upload_fine_kernel(double* __restrict__ uold, const int32
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t dc = ncoarse + (int64_t)active[i >> 3] * 8 + (i & 7);
     const int gs = son[dc];
-    if (gs > 0) restrict_cell(uold, dc, gs, ncell, ncoarse, hp);
+    if (gs > 0) restrict_cell(uold, dc, gs, ncell, ncoarse, hp, nullptr);
   }
 }
 
@@ -791,11 +819,7 @@ static __global__ void __launch_bounds__(NT) set_uold_upload_kernel(
     const int64_t dc = ncoarse + (int64_t)active[i >> 3] * 8 + (i & 7);
     const int gs = do_upload ? son[dc] : 0;
     if (gs > 0) {
-      restrict_cell(uold, dc, gs, ncell, ncoarse, hp);
-      if (next_unew) {
-#pragma unroll
-        for (int v = 0; v < 5; v++) unew[v * ncell + dc] = uold[v * ncell + dc];
-      }
+      restrict_cell(uold, dc, gs, ncell, ncoarse, hp, next_unew ? unew : nullptr);
     } else {
       double u[5];
 #pragma unroll

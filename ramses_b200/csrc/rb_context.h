@@ -147,6 +147,11 @@ struct rb_context {
   int precision = RB_PREC_FP64;
   int device = 0;
   int64_t ncell = 0;
+  // device layout: the cells of oct igrid start at oct0 + 8*(igrid-1), a
+  // variable's array holds dcell values. oct0 and dcell are multiples of 8 and
+  // 16, so that an oct's eight cells of one variable are one aligned 64-byte row
+  int32_t oct0 = 0;
+  int64_t dcell = 0;
   cudaStream_t stream = nullptr;
   cudaMemPool_t table_pool = nullptr;  // the level tables' device buffers (grow-only, kept across re-syncs)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;

@@ -76,7 +76,7 @@ inline int64_t fcell(const rb_context* c, int ind /*1..8*/, int igrid /*1-based*
 inline int64_t dev_of_fortran(const rb_context* c, int64_t icell) {
   if (icell <= c->mp.ncoarse) return icell - 1;
   const int64_t r = icell - 1 - c->mp.ncoarse;
-  return c->mp.ncoarse + (r % c->mp.ngridmax) * 8 + r / c->mp.ngridmax;
+  return c->oct0 + (r % c->mp.ngridmax) * 8 + r / c->mp.ngridmax;
 }
 
 inline uint64_t morton2(uint64_t x, uint64_t y) {
@@ -302,7 +302,7 @@ int ensure_nres6(rb_context* c, Level& L) {
     for (int j = 0; j < 6; j++) {
       const int64_t fcell = c->nbor[(size_t)j * c->mp.ngridmax + (g - 1)];
       const int32_t gn = c->son[fcell - 1];
-      nr[(size_t)i * 6 + j] = gn > 0 ? (int64_t)c->mp.ncoarse + 8 * (int64_t)(gn - 1) : -dev_of_fortran(c, fcell) - 1;
+      nr[(size_t)i * 6 + j] = gn > 0 ? (int64_t)c->oct0 + 8 * (int64_t)(gn - 1) : -dev_of_fortran(c, fcell) - 1;
     }
   }
   RB_TRY(dreserve(c->table_pool, c->stream, &L.d_nres6, &L.cap_nres6, nr.size()));
@@ -762,7 +762,7 @@ int prolong_new_octs(rb_context* c, const std::vector<std::vector<int32_t>>& bor
     RB_TRY(h2d(c, d_octs, octs.data(), octs.size() * 4));
     RB_TRY(h2d(c, d_cells, cells7.data(), cells7.size() * 4));
     rb::prolong_new_octs_kernel<<<(int)((octs.size() + 127) / 128), 128, 0, c->stream>>>(
-        c->d_uold, d_cells, d_octs, (int32_t)octs.size(), c->ncell, c->mp.ncoarse, c->hp);
+        c->d_uold, d_cells, d_octs, (int32_t)octs.size(), c->dcell, c->oct0, c->hp);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(RB_ERR_CUDA, "prolongation of new octs failed: %s", cudaGetErrorString(e));
     RB_CUDA(cudaStreamSynchronize(c->stream));
@@ -1003,7 +1003,7 @@ int sync_tree_impl(rb_context* c, const int32_t* son, const int32_t* father, con
   if (!incremental) {
     RB_TRY(h2d(c, c->d_stage, son, ncell * 4));
     rb::permute_son_kernel<<<grid_for(ncell, 256), 256, 0, c->stream>>>((const int32_t*)c->d_stage, c->d_son, ncell,
-                                                                        c->mp.ncoarse, ngm);
+                                                                        c->mp.ncoarse, c->oct0, ngm);
     RB_CUDA(cudaGetLastError());
     RB_CUDA(cudaStreamSynchronize(c->stream));
   } else if (!son_idx.empty()) {
@@ -1079,10 +1079,10 @@ int set_unew_impl(rb_context* c, int l) {
   const int grid = grid_for((int64_t)L.noct * 8, 256);
   if (c->hp.pressure_fix)
     rb::pf_set_unew_kernel<<<grid, 256, 0, c->stream>>>(c->d_uold, c->d_unew, c->d_divu, c->d_enew, L.d_active, L.noct,
-                                                        c->ncell, c->mp.ncoarse, c->hp.smallr, c->gate);
+                                                        c->dcell, c->oct0, c->hp.smallr, c->gate);
   else
-    rb::copy_octs_kernel<<<grid, 256, 0, c->stream>>>(c->d_uold, c->d_unew, L.d_active, L.noct, c->ncell,
-                                                      c->mp.ncoarse, c->gate);
+    rb::copy_octs_kernel<<<grid, 256, 0, c->stream>>>(c->d_uold, c->d_unew, L.d_active, L.noct, c->dcell,
+                                                      c->oct0, c->gate);
   RB_CUDA(cudaGetLastError());
   return RB_OK;
 }
@@ -1094,7 +1094,7 @@ int pdv_impl(rb_context* c, int l, const double* dt_dev, double dt) {
   int e2;
   const int dx_pow2 = std::frexp(L.dx, &e2) == 0.5;
   rb::pdv_kernel<<<grid_for((int64_t)L.noct * 8, 256), 256, 0, c->stream>>>(
-      c->d_uold, L.d_active, L.d_nres6, L.noct, c->ncell, c->mp.ncoarse, L.dx, dx_pow2, dt_dev, dt, c->hp,
+      c->d_uold, L.d_active, L.d_nres6, L.noct, c->dcell, c->oct0, L.dx, dx_pow2, dt_dev, dt, c->hp,
       c->d_enew, c->gate);
   RB_CUDA(cudaGetLastError());
   return RB_OK;
@@ -1104,7 +1104,7 @@ int pdv_impl(rb_context* c, int l, const double* dt_dev, double dt) {
 int pf_fix_impl(rb_context* c, int l, const double* dt_dev, double dt, int skip_split) {
   Level& L = c->lv[l];
   rb::pf_fix_kernel<<<grid_for((int64_t)L.noct * 8, 256), 256, 0, c->stream>>>(
-      c->d_uold, c->d_divu, c->d_enew, c->d_son, L.d_active, L.noct, c->ncell, c->mp.ncoarse, L.dx, dt_dev, dt,
+      c->d_uold, c->d_divu, c->d_enew, c->d_son, L.d_active, L.noct, c->dcell, c->oct0, L.dx, dt_dev, dt,
       c->hp.smallr, c->hp.beta_fix, skip_split, c->gate);
   RB_CUDA(cudaGetLastError());
   return RB_OK;
@@ -1117,7 +1117,7 @@ int set_uold_impl(rb_context* c, int l) {
   if (!L.noct) return RB_OK;
   if (c->hp.pressure_fix) RB_TRY(pdv_impl(c, l, nullptr, c->dt_godunov[l]));
   rb::copy_octs_kernel<<<grid_for((int64_t)L.noct * 8, 256), 256, 0, c->stream>>>(
-      c->d_unew, c->d_uold, L.d_active, L.noct, c->ncell, c->mp.ncoarse, c->gate);
+      c->d_unew, c->d_uold, L.d_active, L.noct, c->dcell, c->oct0, c->gate);
   RB_CUDA(cudaGetLastError());
   if (c->hp.pressure_fix) RB_TRY(pf_fix_impl(c, l, nullptr, c->dt_godunov[l], 0));
   return RB_OK;
@@ -1137,7 +1137,7 @@ int set_uold_upload_impl(rb_context* c, int l, const double* dt_dev, double dt, 
   auto k = c->precision == RB_PREC_MIXED ? rb::set_uold_upload_kernel<256, true> : rb::set_uold_upload_kernel<256, false>;
   // with a tail: one wave of CTAs, each of which signals its completion once
   k<<<grid_for((int64_t)L.noct * 8, 256, tail ? 148 * 8 : 148 * 32), 256, 0, c->stream>>>(
-      c->d_uold, c->d_unew, c->d_son, L.d_active, L.noct, c->ncell, c->mp.ncoarse, c->hp, do_upload, c->gate,
+      c->d_uold, c->d_unew, c->d_son, L.d_active, L.noct, c->dcell, c->oct0, c->hp, do_upload, c->gate,
       c->d_divu, c->d_enew, L.dx, dt_dev, dt, next_unew, tail ? *tail : none);
   RB_CUDA(cudaGetLastError());
   return RB_OK;
@@ -1148,7 +1148,7 @@ int upload_fine_impl(rb_context* c, int l) {
   Level& L = c->lv[l];
   if (!L.noct || !L.has_refined) return RB_OK;
   rb::upload_fine_kernel<<<grid_for((int64_t)L.noct * 8, 256), 256, 0, c->stream>>>(
-      c->d_uold, c->d_son, L.d_active, L.noct, c->ncell, c->mp.ncoarse, c->hp, c->gate);
+      c->d_uold, c->d_son, L.d_active, L.noct, c->dcell, c->oct0, c->hp, c->gate);
   RB_CUDA(cudaGetLastError());
   return RB_OK;
 }
@@ -1163,7 +1163,7 @@ int boundary_impl(rb_context* c, int l) {
     if (n == 0) continue;
     for (int phase = 0; phase < 2; phase++) {
       rb::boundary_fill_kernel<<<grid_for(n * 8, 256), 256, 0, c->stream>>>(
-          c->d_uold, L.d_bpair + 2 * L.h_boff[ib], n, c->ncell, c->mp.ncoarse, c->btype[ib], c->hp.smallr,
+          c->d_uold, L.d_bpair + 2 * L.h_boff[ib], n, c->dcell, c->oct0, c->btype[ib], c->hp.smallr,
           c->d_bbuf, phase, c->gate);
       RB_CUDA(cudaGetLastError());
     }
@@ -1184,7 +1184,7 @@ int sync_oct(rb_context* c) {
   Level& L = c->lv[c->finest];
   const int64_t vstr = (int64_t)c->dnx * c->dny * c->dnz;
   rb::dense_to_oct_kernel<<<grid_for((int64_t)L.noct * 8, 256), 256, 0, c->stream>>>(
-      c->d_dense[c->dense_cur], c->d_uold, L.d_active, c->d_cbase, L.noct, c->ncell, c->mp.ncoarse, c->dnx,
+      c->d_dense[c->dense_cur], c->d_uold, L.d_active, c->d_cbase, L.noct, c->dcell, c->oct0, c->dnx,
       c->dny, vstr);
   RB_CUDA(cudaGetLastError());
   for (int l = c->finest - 1; l >= 1; l--) RB_TRY(upload_fine_impl(c, l));
@@ -1275,9 +1275,9 @@ rb::TileArgs tile_args(rb_context* c, Level& L, double dt) {
   a.divu = c->d_divu;    // null unless pressure_fix
   a.enew = c->d_enew;
   a.corr_tmp = L.d_corr_tmp;
-  a.ncell = c->ncell;
+  a.ncell = c->dcell;
   a.ninterp8 = (int64_t)L.ninterp * 8;
-  a.ncoarse = c->mp.ncoarse;
+  a.ncoarse = c->oct0;
   a.ntile = L.ntile;
   a.has_refined = L.has_refined;
   int e2;
@@ -1306,10 +1306,10 @@ int interp_impl(rb_context* c, Level& L, const double* gate) {
   if (!L.ninterp) return RB_OK;
   const unsigned nb = (unsigned)((L.ninterp + 127) / 128);
   if (c->hp.interpol_var == 0)
-    rb::interp_blocks_var_kernel<<<dim3(nb, 5), 128, 0, c->stream>>>(c->d_uold, L.d_interp7, L.ninterp, c->ncell,
+    rb::interp_blocks_var_kernel<<<dim3(nb, 5), 128, 0, c->stream>>>(c->d_uold, L.d_interp7, L.ninterp, c->dcell,
                                                                      L.d_interp_buf, c->hp.interpol_type, gate);
   else
-    rb::interp_blocks_kernel<<<nb, 128, 0, c->stream>>>(c->d_uold, L.d_interp7, L.ninterp, c->ncell, L.d_interp_buf,
+    rb::interp_blocks_kernel<<<nb, 128, 0, c->stream>>>(c->d_uold, L.d_interp7, L.ninterp, c->dcell, L.d_interp_buf,
                                                         c->hp, gate);
   RB_CUDA(cudaGetLastError());
   return RB_OK;
@@ -1343,7 +1343,7 @@ int godunov_impl(rb_context* c, int l, double dt, bool timed, const double* dt_d
   if (L.ntgt) {
     const int64_t nval = (int64_t)L.ntgt * (c->d_divu ? 7 : 5);
     rb::apply_corrections_kernel<<<(unsigned)((nval + 127) / 128), 128, 0, c->stream>>>(
-        c->d_unew, L.d_tgt, L.d_tgt_off, L.d_contrib, L.ntgt, L.d_corr_flux, c->ncell, c->gate, c->d_divu, c->d_enew,
+        c->d_unew, L.d_tgt, L.d_tgt_off, L.d_contrib, L.ntgt, L.d_corr_flux, c->dcell, c->gate, c->d_divu, c->d_enew,
         L.d_corr_tmp);
     RB_CUDA(cudaGetLastError());
   }
@@ -1358,7 +1358,7 @@ int courant_impl(rb_context* c, int l, double* dt_io, double* mass, double* ekin
   const int nblk = grid_for((int64_t)L.noct * 8, nt, 148 * 8);
   RB_TRY(ensure_partial(c, nblk));
   auto k = c->precision == RB_PREC_MIXED ? rb::courant_partial_kernel<256, true> : rb::courant_partial_kernel<256, false>;
-  k<<<nblk, nt, 0, c->stream>>>(c->d_uold, c->d_son, L.d_active, L.noct, c->ncell, c->mp.ncoarse, L.dx, c->hp,
+  k<<<nblk, nt, 0, c->stream>>>(c->d_uold, c->d_son, L.d_active, L.noct, c->dcell, c->oct0, L.dx, c->hp,
                                 c->d_partial, c->gate, with_set_unew ? c->d_unew : nullptr,
                                 with_set_unew ? c->d_divu : nullptr, with_set_unew ? c->d_enew : nullptr);
   RB_CUDA(cudaGetLastError());
@@ -1492,8 +1492,8 @@ int sched_impl(rb_context* c, const std::vector<uint16_t>& ops) {
 int level_cfl_impl(rb_context* c, int l, const double* u, double* unew, const rb::CflTail& tail) {
   Level& L = c->lv[l];
   auto k = c->precision == RB_PREC_MIXED ? rb::level_cfl_kernel<256, true> : rb::level_cfl_kernel<256, false>;
-  k<<<grid_for((int64_t)L.noct * 8, 256, 148 * 8), 256, 0, c->stream>>>(u, c->d_son, L.d_active, L.noct, c->ncell,
-                                                                       c->mp.ncoarse, c->hp, unew, c->gate, tail);
+  k<<<grid_for((int64_t)L.noct * 8, 256, 148 * 8), 256, 0, c->stream>>>(u, L.has_refined ? c->d_son : nullptr, L.d_active, L.noct, c->dcell,
+                                                                       c->oct0, c->hp, unew, c->gate, tail);
   RB_CUDA(cudaGetLastError());
   return RB_OK;
 }
@@ -1715,6 +1715,8 @@ int rb_create(const rb_hydro_params* hp, const rb_mesh_params* mp, int precision
   c->mp = *mp;
   c->precision = precision;
   c->ncell = (int64_t)mp->ncoarse + 8 * (int64_t)mp->ngridmax;
+  c->oct0 = (mp->ncoarse + 7) / 8 * 8;
+  c->dcell = ((int64_t)c->oct0 + 8 * (int64_t)mp->ngridmax + 15) / 16 * 16;
   auto bail = [&](int rc) { rb_destroy(c); return rc; };
   if (cudaGetDevice(&c->device) != cudaSuccess) return bail(fail(RB_ERR_NO_DEVICE, "cudaGetDevice failed"));
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1736,22 +1738,22 @@ int rb_create(const rb_hydro_params* hp, const rb_mesh_params* mp, int precision
       return bail(fail(RB_ERR_CUDA, "memory pool set-up failed"));
   }
   int rc;
-  if ((rc = dalloc(&c->d_uold, (size_t)c->ncell * 5)) || (rc = dalloc(&c->d_unew, (size_t)c->ncell * 5)) ||
-      (rc = dalloc(&c->d_son, (size_t)c->ncell)) ||
-      (rc = dalloc(&c->d_stage, (size_t)c->ncell * 5)) || (rc = dalloc(&c->d_red, 8)) ||
+  if ((rc = dalloc(&c->d_uold, (size_t)c->dcell * 5)) || (rc = dalloc(&c->d_unew, (size_t)c->dcell * 5)) ||
+      (rc = dalloc(&c->d_son, (size_t)c->dcell)) ||
+      (rc = dalloc(&c->d_stage, (size_t)c->dcell * 5)) || (rc = dalloc(&c->d_red, 8)) ||
       (rc = dalloc(&c->d_clock, 8)) || (rc = dalloc(&c->d_sched, RB_S_SIZE)) || (rc = dalloc(&c->d_cfl, 2)))
     return bail(rc);
   if (c->hp.pressure_fix) {
-    if ((rc = dalloc(&c->d_divu, (size_t)c->ncell)) || (rc = dalloc(&c->d_enew, (size_t)c->ncell))) return bail(rc);
-    if (cudaMemsetAsync(c->d_divu, 0, (size_t)c->ncell * sizeof(double), c->stream) != cudaSuccess ||
-        cudaMemsetAsync(c->d_enew, 0, (size_t)c->ncell * sizeof(double), c->stream) != cudaSuccess)
+    if ((rc = dalloc(&c->d_divu, (size_t)c->dcell)) || (rc = dalloc(&c->d_enew, (size_t)c->dcell))) return bail(rc);
+    if (cudaMemsetAsync(c->d_divu, 0, (size_t)c->dcell * sizeof(double), c->stream) != cudaSuccess ||
+        cudaMemsetAsync(c->d_enew, 0, (size_t)c->dcell * sizeof(double), c->stream) != cudaSuccess)
       return bail(fail(RB_ERR_CUDA, "initialising device buffers failed"));
   }
   if (cudaMallocHost((void**)&c->h_red, 8 * sizeof(double)) != cudaSuccess ||
       cudaMallocHost((void**)&c->h_sched, RB_S_SIZE * sizeof(double)) != cudaSuccess)
     return bail(fail(RB_ERR_NOMEM, "pinned allocation failed"));
-  if (cudaMemsetAsync(c->d_uold, 0, (size_t)c->ncell * 5 * sizeof(double), c->stream) != cudaSuccess ||
-      cudaMemsetAsync(c->d_unew, 0, (size_t)c->ncell * 5 * sizeof(double), c->stream) != cudaSuccess ||
+  if (cudaMemsetAsync(c->d_uold, 0, (size_t)c->dcell * 5 * sizeof(double), c->stream) != cudaSuccess ||
+      cudaMemsetAsync(c->d_unew, 0, (size_t)c->dcell * 5 * sizeof(double), c->stream) != cudaSuccess ||
       cudaMemsetAsync(c->d_clock, 0, 8 * sizeof(double), c->stream) != cudaSuccess ||
       cudaMemsetAsync(c->d_cfl, 0, 2 * sizeof(unsigned long long), c->stream) != cudaSuccess ||
       cudaStreamSynchronize(c->stream) != cudaSuccess)
@@ -1839,16 +1841,16 @@ int rb_make_boundary_hydro(rb_context* c, int l) {
 static int upload_impl(rb_context* c, const double* h, double* d) {
   if (!c || !h) return fail(RB_ERR_INVALID, "null argument");
   RB_CUDA(cudaMemcpyAsync(c->d_stage, h, (size_t)c->ncell * 5 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  rb::permute_f2d_kernel<<<grid_for(c->ncell, 256), 256, 0, c->stream>>>(c->d_stage, d, c->ncell, c->mp.ncoarse,
-                                                                            c->mp.ngridmax, 5);
+  rb::permute_f2d_kernel<<<grid_for(c->ncell, 256), 256, 0, c->stream>>>(c->d_stage, d, c->ncell, c->dcell, c->mp.ncoarse,
+                                                                         c->oct0, c->mp.ngridmax, 5);
   RB_CUDA(cudaGetLastError());
   RB_CUDA(cudaStreamSynchronize(c->stream));
   return RB_OK;
 }
 static int download_impl(rb_context* c, const double* d, double* h) {
   if (!c || !h) return fail(RB_ERR_INVALID, "null argument");
-  rb::permute_d2f_kernel<<<grid_for(c->ncell * 5, 256), 256, 0, c->stream>>>(d, c->d_stage, c->ncell, c->mp.ncoarse,
-                                                                            c->mp.ngridmax, 5);
+  rb::permute_d2f_kernel<<<grid_for(c->ncell * 5, 256), 256, 0, c->stream>>>(d, c->d_stage, c->ncell, c->dcell,
+                                                                             c->mp.ncoarse, c->oct0, c->mp.ngridmax, 5);
   RB_CUDA(cudaGetLastError());
   RB_CUDA(cudaMemcpyAsync(h, c->d_stage, (size_t)c->ncell * 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   RB_CUDA(cudaStreamSynchronize(c->stream));
@@ -1924,7 +1926,7 @@ int rb_upload_level_state(rb_context* c, int ilevel, const double* uold) {
   if (L.noct == 0) return RB_OK;
   RB_TRY(level_rows_copy(c, ilevel, const_cast<double*>(uold), true));
   rb::permute_level_kernel<true><<<grid_for((int64_t)L.noct * 8, 256), 256, 0, c->stream>>>(
-      c->d_stage, c->d_uold, L.d_active, L.noct, c->ncell, c->mp.ncoarse, c->mp.ngridmax);
+      c->d_stage, c->d_uold, L.d_active, L.noct, c->ncell, c->dcell, c->mp.ncoarse, c->oct0, c->mp.ngridmax);
   RB_CUDA(cudaGetLastError());
   RB_CUDA(cudaStreamSynchronize(c->stream));
   oct_changed(c);
@@ -1937,7 +1939,7 @@ int rb_download_level_state(rb_context* c, int ilevel, double* uold) {
   Level& L = c->lv[ilevel];
   if (L.noct == 0) return RB_OK;
   rb::permute_level_kernel<false><<<grid_for((int64_t)L.noct * 8, 256), 256, 0, c->stream>>>(
-      c->d_stage, c->d_uold, L.d_active, L.noct, c->ncell, c->mp.ncoarse, c->mp.ngridmax);
+      c->d_stage, c->d_uold, L.d_active, L.noct, c->ncell, c->dcell, c->mp.ncoarse, c->oct0, c->mp.ngridmax);
   RB_CUDA(cudaGetLastError());
   RB_TRY(level_rows_copy(c, ilevel, uold, false));
   RB_CUDA(cudaStreamSynchronize(c->stream));
@@ -2003,7 +2005,7 @@ int rb_download_pressure_fix(rb_context* c, double* divu, double* enew) {
   if (!c->hp.pressure_fix) return fail(RB_ERR_STATE, "the context was created without pressure_fix");
   for (int k = 0; k < 2; k++) {
     rb::permute_d2f_kernel<<<grid_for(c->ncell, 256), 256, 0, c->stream>>>(
-        k == 0 ? c->d_divu : c->d_enew, c->d_stage, c->ncell, c->mp.ncoarse, c->mp.ngridmax, 1);
+        k == 0 ? c->d_divu : c->d_enew, c->d_stage, c->ncell, c->dcell, c->mp.ncoarse, c->oct0, c->mp.ngridmax, 1);
     RB_CUDA(cudaGetLastError());
     RB_CUDA(cudaMemcpyAsync(k == 0 ? divu : enew, c->d_stage, (size_t)c->ncell * sizeof(double),
                             cudaMemcpyDeviceToHost, c->stream));
@@ -2119,7 +2121,7 @@ int rb_hydro_flag(rb_context* c, int l, const rb_refine_params* rp, int32_t* fla
     c->flag_cap = n;
   }
   rb::hydro_flag_kernel<<<grid_for(n, 256), 256, 0, c->stream>>>(c->d_uold, c->d_son, L.d_active, L.d_nbor6, L.noct,
-                                                                 c->ncell, c->mp.ncoarse, c->hp, *rp, c->d_flag);
+                                                                 c->dcell, c->oct0, c->hp, *rp, c->d_flag);
   RB_CUDA(cudaGetLastError());
   std::vector<uint8_t> f((size_t)n);
   RB_CUDA(cudaMemcpyAsync(f.data(), c->d_flag, (size_t)n, cudaMemcpyDeviceToHost, c->stream));
@@ -2254,7 +2256,7 @@ int rb_set_tile_shape(rb_context* c, int l, int shape) {
     L.shape = s;
     RB_TRY(build_level_tables(c, l, c->idx));
     RB_TRY(interp_impl(c, L, nullptr));
-    RB_CUDA(cudaMemcpyAsync(c->d_stage, keep_unew, (size_t)c->ncell * 5 * sizeof(double), cudaMemcpyDeviceToDevice,
+    RB_CUDA(cudaMemcpyAsync(c->d_stage, keep_unew, (size_t)c->dcell * 5 * sizeof(double), cudaMemcpyDeviceToDevice,
                             c->stream));
     c->d_unew = c->d_stage;
     rb::TileArgs a = tile_args(c, L, 1e-30);
@@ -2304,8 +2306,8 @@ static int uniform_run_tiles(rb_context* c, int nsteps, int use_graph, double* t
     // newdt_fine + courant_fine on the starting state
     const int nblk = grid_for((int64_t)L.noct * 8, 256, 148 * 8);
     RB_TRY(ensure_partial(c, nblk));
-    rb::courant_partial_kernel<256><<<nblk, 256, 0, c->stream>>>(c->d_uold, c->d_son, L.d_active, L.noct, c->ncell,
-                                                                c->mp.ncoarse, L.dx, c->hp, c->d_partial, nullptr);
+    rb::courant_partial_kernel<256><<<nblk, 256, 0, c->stream>>>(c->d_uold, c->d_son, L.d_active, L.noct, c->dcell,
+                                                                c->oct0, L.dx, c->hp, c->d_partial, nullptr);
     RB_CUDA(cudaGetLastError());
     rb::reduce_partials_kernel<<<1, RB_RED_NT, 0, c->stream>>>(c->d_partial, nblk, dt_max, dt0, 1, c->d_red, 0);
     RB_CUDA(cudaGetLastError());
@@ -2423,7 +2425,7 @@ static int uniform_run_dense(rb_context* c, int nsteps, int use_graph, double* t
   if (!c->dense_valid) {
     RB_TRY(sync_oct(c));
     rb::oct_to_dense_kernel<<<grid_for((int64_t)L.noct * 8, 256), 256, 0, c->stream>>>(
-        c->d_uold, c->d_dense[c->dense_cur], L.d_active, c->d_cbase, L.noct, c->ncell, c->mp.ncoarse, c->dnx,
+        c->d_uold, c->d_dense[c->dense_cur], L.d_active, c->d_cbase, L.noct, c->dcell, c->oct0, c->dnx,
         c->dny, vstr);
     RB_CUDA(cudaGetLastError());
     c->dense_valid = true;
@@ -2432,8 +2434,8 @@ static int uniform_run_dense(rb_context* c, int nsteps, int use_graph, double* t
   RB_TRY(ensure_partial(c, grid_for((int64_t)L.noct * 8, 256, 148 * 8)));
   if (!c->clock_valid) {
     const int nblk = grid_for((int64_t)L.noct * 8, 256, 148 * 8);
-    rb::courant_partial_kernel<256><<<nblk, 256, 0, c->stream>>>(c->d_uold, c->d_son, L.d_active, L.noct, c->ncell,
-                                                                c->mp.ncoarse, L.dx, c->hp, c->d_partial, nullptr);
+    rb::courant_partial_kernel<256><<<nblk, 256, 0, c->stream>>>(c->d_uold, c->d_son, L.d_active, L.noct, c->dcell,
+                                                                c->oct0, L.dx, c->hp, c->d_partial, nullptr);
     RB_CUDA(cudaGetLastError());
     rb::reduce_partials_kernel<<<1, RB_RED_NT, 0, c->stream>>>(c->d_partial, nblk, dt_max, dt0, 1, c->d_red, 0);
     RB_CUDA(cudaGetLastError());
@@ -2548,7 +2550,7 @@ int rb_autotune_uniform(rb_context* c, int* shape_out, int* hz_out, float* ms_ou
     RB_TRY(sync_oct(c));
     const int64_t vstr = (int64_t)c->dnx * c->dny * c->dnz;
     rb::oct_to_dense_kernel<<<grid_for((int64_t)L.noct * 8, 256), 256, 0, c->stream>>>(
-        c->d_uold, c->d_dense[c->dense_cur], L.d_active, c->d_cbase, L.noct, c->ncell, c->mp.ncoarse, c->dnx,
+        c->d_uold, c->d_dense[c->dense_cur], L.d_active, c->d_cbase, L.noct, c->dcell, c->oct0, c->dnx,
         c->dny, vstr);
     RB_CUDA(cudaGetLastError());
     c->dense_valid = true;
@@ -2559,8 +2561,8 @@ int rb_autotune_uniform(rb_context* c, int* shape_out, int* hz_out, float* ms_ou
     double d = c->mp.boxlen / c->hp.smallc;
     const int nblk = grid_for((int64_t)L.noct * 8, 256, 148 * 8);
     RB_TRY(ensure_partial(c, nblk));
-    rb::courant_partial_kernel<256><<<nblk, 256, 0, c->stream>>>(c->d_uold, c->d_son, L.d_active, L.noct, c->ncell,
-                                                                c->mp.ncoarse, L.dx, c->hp, c->d_partial, nullptr);
+    rb::courant_partial_kernel<256><<<nblk, 256, 0, c->stream>>>(c->d_uold, c->d_son, L.d_active, L.noct, c->dcell,
+                                                                c->oct0, L.dx, c->hp, c->d_partial, nullptr);
     RB_CUDA(cudaGetLastError());
     rb::reduce_partials_kernel<<<1, RB_RED_NT, 0, c->stream>>>(c->d_partial, nblk, d, c->hp.courant_factor * L.dx / c->hp.smallc, 1, c->d_red + 4, 0);
     RB_CUDA(cudaGetLastError());
