@@ -19,6 +19,8 @@
 // Compiled with --fmad=false.
 #include <chrono>
 #include <deque>
+#include <functional>
+#include <queue>
 
 #include "rb_context.h"
 #include "serve_kernels.cuh"
@@ -66,6 +68,7 @@ struct Request {
 };
 
 constexpr int kMaxSlots = 1 << 16;  // dense problems resident at once
+constexpr int kBatchCtasPerSm = 2;  // register budget of the batched kernels (RB_BATCH_LAUNCH)
 
 }  // namespace
 
@@ -102,6 +105,7 @@ struct rb_server {
   std::deque<int64_t> done_pending;  // completed ids not yet returned
   int64_t total_updates = 0;
   int64_t rounds_launched = 0, batch_launches = 0;
+  std::vector<int64_t> plan_ids;  // members (launch order) that the z extents were chosen for
 };
 
 namespace {
@@ -115,14 +119,62 @@ int64_t tree_bytes(const rb_mesh_params& mp) {
   return ncell * (3 * 5 * 8 + 4) + (int64_t)mp.ngridmax * 96 + (4 << 20);
 }
 
-// the longest z extent (power of two <= 64 dividing nz) that still gives the
-// problem at least 16 work items
-int pick_hz(int nx, int ny, int nz, int tx, int ty) {
-  const int cols = (nx / tx) * (ny / ty);
-  int hz = 64;
-  while (hz > 8 && (nz % hz != 0 || cols * (nz / hz) < 16)) hz >>= 1;
+// the longest z extent of a work item (a power of two <= cap) dividing nz
+int z_extent(int nz, int cap) {
+  int hz = cap;
   while (hz > 2 && nz % hz != 0) hz >>= 1;
   return hz;
+}
+
+// The z extents of a round: the cap on every problem's extent for which the
+// round's items, dealt in launch order to the CTAs that fit at once, end first
+// (an item of hz planes streams hz + 2 and has a prologue of about two). A
+// fixed extent of at least 16 items per problem left a small batch with a few
+// long items: two 32^3 problems 20 planes where extent 2 takes 6, four 64^3
+// ones 68 against 36; 24 problems of 32^3 and 64^3 108 against 96. The results
+// do not depend on the extents, and the plan changes only with the members.
+void plan_round(rb_server* s) {
+  std::vector<int64_t> ids;
+  ids.reserve(s->dense.size());
+  for (const Request* r : s->dense) ids.push_back(r->id);
+  if (ids == s->plan_ids) return;
+  s->plan_ids.swap(ids);
+  const int tx = rb::kStreamShapes[s->shape][0], ty = rb::kStreamShapes[s->shape][1];
+  const int slots = 148 * kBatchCtasPerSm;
+  auto items = [&](const Request* r, int hz) { return (r->nx / tx) * (r->ny / ty) * (r->nz / hz); };
+  int best_cap = 64;
+  double best = HUGE_VAL;
+  for (int cap = 64; cap >= 2; cap >>= 1) {
+    int64_t n = 0, planes = 0;
+    int longest = 0;
+    for (const Request* r : s->dense) {
+      const int hz = z_extent(r->nz, cap), k = items(r, hz);
+      n += k;
+      planes += (int64_t)k * (hz + 4);
+      longest = std::max(longest, hz + 4);
+    }
+    double t = (double)planes / slots + longest;  // many items: the tail is at most one of them
+    if (n <= 4 * slots) {
+      std::priority_queue<int, std::vector<int>, std::greater<int>> free_at;
+      for (int i = 0; i < slots; i++) free_at.push(0);
+      int end = 0;
+      for (const Request* r : s->dense) {
+        const int hz = z_extent(r->nz, cap);
+        for (int k = items(r, hz); k > 0; k--) {
+          const int e = free_at.top() + hz + 4;
+          free_at.pop();
+          free_at.push(e);
+          end = std::max(end, e);
+        }
+      }
+      t = end;
+    }
+    if (t < best) { best = t; best_cap = cap; }
+  }
+  for (Request* r : s->dense) {
+    r->hz = z_extent(r->nz, best_cap);
+    r->items = items(r, r->hz);
+  }
 }
 
 int grow_round_buffers(rb_server* s, int nprob) {
@@ -248,6 +300,7 @@ int launch_round(rb_server* s) {
   const int k = s->round & 1;
   s->round_members[k].clear();
   int nitems = 0;
+  plan_round(s);
   for (Request* r : s->dense) nitems += r->items;
   const int nprob = (int)s->dense.size();
   if (nprob) {
@@ -522,8 +575,6 @@ int rb_server_submit_dense(rb_server* s, int32_t nx, int32_t ny, int32_t nz, dou
     delete r;
     return fail(RB_ERR_INVALID, "dense problems are cubes of cubic cells (nx=ny=nz)");
   }
-  r->hz = pick_hz(nx, ny, nz, tx, ty);
-  r->items = (nx / tx) * (ny / ty) * (nz / r->hz);
   r->bytes = dense_bytes((int64_t)nx * ny * nz);
   if (r->bytes > s->budget) {
     delete r;
