@@ -749,7 +749,7 @@ def main():
                                                "(profiles/opcount_hllc_moncen_turb.md)"},
             "cpu_baseline": cpu,
             "clocks": clk_sum,
-            "gpu_launches": 2 * args.steps,
+            "gpu_launches": args.steps,  # one step kernel per step (it advances the clock itself)
             "fp64": {"value": f64_value, "ms_per_step": f64_ms / args.steps, "kernel_ms": f64_kern,
                      "kernel": f64_kernel,
                      "roofline_frac": BYTES_PER_CELL_UPDATE * cells / (f64_kern / 1e3) / 1e9 / peak,
