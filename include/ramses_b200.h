@@ -189,7 +189,9 @@ int rb_cell_updates(rb_context *ctx, int64_t *out);
 
 /* Choose the tile shape of level ilevel's godunov kernel: shape >= 0 forces
  * one (see rb_tile_shape_info), shape < 0 times every shape on the current
- * state and keeps the fastest (the state is left unchanged). */
+ * state and keeps the fastest (the state is left unchanged). Where the octs of
+ * a periodic axis are not a multiple of the forced shape's, the next smaller
+ * shape that divides them is taken (rb_get_tile_shape tells which). */
 int rb_set_tile_shape(rb_context *ctx, int ilevel, int shape);
 int rb_get_tile_shape(rb_context *ctx, int ilevel, int *shape);
 int rb_tile_shape_info(int shape, int *tx, int *ty, int *tz, int *nthreads);

@@ -249,16 +249,40 @@ struct ParError {
   int report() const { return set.load() ? fail(code, "%s", msg.c_str()) : RB_OK; }
 };
 
+// Octs of a level along each axis of the coarse grid, and the axes with
+// physical boundaries.
+struct LevelAxes {
+  int64_t noct[3];
+  bool bounded[3] = {false, false, false};
+};
+LevelAxes level_axes(const rb_context* c, int l) {
+  LevelAxes a;
+  const int32_t n[3] = {c->mp.nx, c->mp.ny, c->mp.nz};
+  for (int d = 0; d < 3; d++) a.noct[d] = (int64_t)n[d] << (l - 1);
+  for (int32_t bt : c->btype) a.bounded[(bt % 10 - 1) / 2] = true;
+  return a;
+}
 // With physical boundaries a tile must not hold both octs of the box and
 // boundary octs: along a bounded axis the tile's octs must divide the
 // 2^(l-1) octs of one coarse cell.
+bool shape_clears_boundary(const rb_context* c, int l, int shape) {
+  const rb::TileShape sh = rb::kTileShapes[shape];
+  const LevelAxes ax = level_axes(c, l);
+  const int to[3] = {sh.tx / 2, sh.ty / 2, sh.tz / 2};
+  for (int d = 0; d < 3; d++)
+    if (ax.bounded[d] && ((int64_t)1 << (l - 1)) % to[d] != 0) return false;
+  return true;
+}
+// Along every axis the tile's octs must divide the level's: a tile reaching
+// past a periodic axis would hold an oct a second time (in one tile or in
+// two), and both copies would update its unew.
 bool shape_fits(const rb_context* c, int l, int shape) {
   const rb::TileShape sh = rb::kTileShapes[shape];
-  const int64_t h = (int64_t)1 << (l - 1);
+  const LevelAxes ax = level_axes(c, l);
   const int to[3] = {sh.tx / 2, sh.ty / 2, sh.tz / 2};
-  for (int32_t bt : c->btype)
-    if (h % to[(bt % 10 - 1) / 2] != 0) return false;
-  return true;
+  for (int d = 0; d < 3; d++)
+    if (ax.noct[d] % to[d] != 0) return false;
+  return shape_clears_boundary(c, l, shape);
 }
 
 // Default tile shape of a level. 8x8x4 cells trace the fewest slab cells per
@@ -384,8 +408,10 @@ int build_level_tables(rb_context* c, int l, const std::vector<OctIndex>& idx) {
   pc.mark("free");
   if (L.noct == 0) return RB_OK;
   if (L.shape < 0 || !L.shape_user) L.shape = default_shape(c, l, L);
-  if (!shape_fits(c, l, L.shape))
+  if (!shape_clears_boundary(c, l, L.shape))
     return fail(RB_ERR_INVALID, "level %d: tile shape %d spans the box face and the boundary layer", l, L.shape);
+  // a chosen shape wider than a periodic level gives way to the next smaller one (one oct always fits)
+  while (!shape_fits(c, l, L.shape)) L.shape--;
   const rb::TileShape sh = rb::kTileShapes[L.shape];
   const int TOX = sh.tx / 2, TOY = sh.ty / 2, TOZ = sh.tz / 2;
   const int BX = TOX + 2, BY = TOY + 2, BZ = TOZ + 2, NBLK = BX * BY * BZ;
@@ -446,8 +472,10 @@ int build_level_tables(rb_context* c, int l, const std::vector<OctIndex>& idx) {
   // stencil box; an absent block that an oct of the tile needs is marked
   // with its father cell f as -1 - f (prolongation entries are numbered in
   // pass 2)
+  std::atomic<int64_t> held{0};  // octs inside the tiles
   parallel_for(L.ntile, 256, [&](int64_t t0, int64_t t1) {
     std::vector<char> inner((size_t)TOX * TOY * TOZ);
+    int64_t n_inner = 0;
     for (int64_t t = t0; t < t1 && !perr.set.load(); t++) {
       const int64_t ox0 = tiles[t].second[0] * TOX, oy0 = tiles[t].second[1] * TOY, oz0 = tiles[t].second[2] * TOZ;
       int32_t* B = &blk[(size_t)t * NBLK];
@@ -480,6 +508,7 @@ int build_level_tables(rb_context* c, int l, const std::vector<OctIndex>& idx) {
               return;
             }
             inner[x + TOX * (y + TOY * z)] = g >= 0;
+            n_inner += g >= 0;
           }
       for (int bz = 0; bz < BZ; bz++)
         for (int by = 0; by < BY; by++)
@@ -500,8 +529,12 @@ int build_level_tables(rb_context* c, int l, const std::vector<OctIndex>& idx) {
             code = (int32_t)(-1 - f);
           }
     }
+    held += n_inner;
   });
   RB_TRY(perr.report());
+  // every oct is inside the tile of its position, so inside no other when the counts agree
+  if (held.load() != L.noct)
+    return fail(RB_ERR_TREE, "level %d: the tiles hold %lld octs of %d", l, (long long)held.load(), L.noct);
   pc.mark("pass1");
   // pass 2: one prolongation entry per distinct father cell, numbered in the
   // order of first use (tile order, so that a tile's entries lie together in
