@@ -25,7 +25,9 @@
 // What bounds it: instruction issue (FP32-mixed) and the latency of the FP64
 // chains (drop-in), so what counts is instructions per cell and CTAs in
 // flight. States are packed for 128-bit shared accesses, and only one of a
-// face's two states passes through shared memory.
+// face's two states passes through shared memory. The variant that reads the
+// scheme at run time differs (kBothStates): it holds every solver and both
+// predictors, whose registers are worth more than the shared traffic.
 #pragma once
 #include <cstdint>
 #include <type_traits>
@@ -182,30 +184,44 @@ template <> struct States<double> {
   }
 };
 
+// The run-time scheme variant passes both states of every face and the lower
+// fluxes of a cell through shared memory, traces cells and slab cells as one
+// list of items, a direction at a time, and solves the faces as another list,
+// through one copy of the predictors and solvers. With the compiled variants'
+// layout (15 states, 15 fluxes and six solver copies per thread) the FP64
+// variant needed 202-236 registers, spilled 650 bytes at its 128 and took 7.7 ms where
+// this takes 4.2 (acoustic, two coarse steps of levels 6-8; slope type 3 8.3
+// against 4.9); FP32-mixed slope type 3 2.91 against 2.83 ms, and a level of 512 octs
+// 12.3 against 15.2 us.
+template <typename R, int RS>
+constexpr bool kBothStates = RS == 0;
+
 // dynamic shared memory: the stencil's primitive states, reused for the face
 // fluxes once they are traced; the lower cell's state at every face; the
-// upper slab's state at the far faces; block codes; flags
-template <typename R, int TX, int TY, int TZ>
+// upper slab's state at the far faces (BOTH: the upper cell's at every face);
+// block codes; flags
+template <typename R, int TX, int TY, int TZ, bool BOTH>
 struct TileSmem {
   using G = TileGeom<TX, TY, TZ>;
   static constexpr size_t Q = 0;
   static constexpr size_t L = (States<R>::bytes(G::NS > G::NF ? G::NS : G::NF) + 15) & ~(size_t)15;
   static constexpr size_t U = L + ((States<R>::bytes(G::NF) + 15) & ~(size_t)15);
-  static constexpr size_t BLK = U + ((States<R>::bytes(G::NU) + 15) & ~(size_t)15);
+  static constexpr int NUP = BOTH ? G::NF : G::NU;
+  static constexpr size_t BLK = U + ((States<R>::bytes(NUP) + 15) & ~(size_t)15);
   static constexpr size_t OK = BLK + sizeof(int32_t) * (size_t)G::NBLK;
   static constexpr size_t SIZE = OK + (size_t)((G::NS + 15) & ~15);
 };
-template <typename R, int TX, int TY, int TZ>
+template <typename R, int TX, int TY, int TZ, bool BOTH>
 constexpr size_t tile_smem_bytes() {
-  return TileSmem<R, TX, TY, TZ>::SIZE;
+  return TileSmem<R, TX, TY, TZ, BOTH>::SIZE;
 }
 
 // Traced face states of one cell from its state q0 and its neighbours in q
 // (stencil slot s): sp[d] at the lower, sm[d] at the upper face of direction d,
-// for the directions of mask.
-template <typename R, int TX, int TY, int TZ, int RS, int ST>
+// for the directions of mask, each handed to put(d, sp, sm).
+template <typename R, int TX, int TY, int TZ, int RS, int ST, typename Put>
 __device__ __forceinline__ void trace_slot(const States<R>& q, int s, const Consts<R>& c, int slope_type,
-                                           const R dtd[3], unsigned mask, Prim<R> sp[3], Prim<R> sm[3]) {
+                                           const R dtd[3], unsigned mask, Put&& put) {
   using G = TileGeom<TX, TY, TZ>;
   constexpr int st[3] = {1, G::SX, G::SX * G::SY};
   const Prim<R> q0 = q.get(s);
@@ -226,8 +242,7 @@ __device__ __forceinline__ void trace_slot(const States<R>& q, int s, const Cons
       if (!(mask & (1u << d))) continue;
       float P[5], M[5];
       face_pair(h, hd, d, q0.r, c.smallr, P, M);
-      sp[d] = Prim<float>{P[0], P[1], P[2], P[3], P[4]};
-      sm[d] = Prim<float>{M[0], M[1], M[2], M[3], M[4]};
+      put(d, Prim<float>{P[0], P[1], P[2], P[3], P[4]}, Prim<float>{M[0], M[1], M[2], M[3], M[4]});
     }
   } else {
     R dq[5][3];
@@ -280,9 +295,30 @@ __device__ __forceinline__ void trace_slot(const States<R>& q, int s, const Cons
         dq[v][0] = slop * dq[v][0]; dq[v][1] = slop * dq[v][1]; dq[v][2] = slop * dq[v][2];
       }
     }
-    trace_sel<R, RS, ST>(q0, dq, c, dtd, sp, sm, mask);
+    Prim<R> sp[3], sm[3];
+    if constexpr (kBothStates<R, RS>) {
+      // a direction at a time: the two predictors meet with one pair of states live, not three
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        if (!(mask & (1u << d))) continue;
+        trace_sel<R, RS, ST>(q0, dq, c, dtd, sp, sm, 1u << d);
+        put(d, sp[d], sm[d]);
+      }
+    } else {
+      trace_sel<R, RS, ST>(q0, dq, c, dtd, sp, sm, mask);
+#pragma unroll
+      for (int d = 0; d < 3; d++)
+        if (mask & (1u << d)) put(d, sp[d], sm[d]);
+    }
   }
 }
+
+// A direction known at compile time, as an argument.
+template <int D>
+struct Axis {
+  static constexpr int value = D;
+  __host__ __device__ constexpr operator int() const { return D; }
+};
 
 // RS (Riemann solver) and ST (slope type) fix the scheme at compile time;
 // RS = 0 / ST = -1 read it from a.hp at run time. PF: pressure_fix, the
@@ -293,7 +329,8 @@ __device__ __forceinline__ void trace_slot(const States<R>& q, int s, const Cons
 template <typename R, int TX, int TY, int TZ, int NT, int MINB, int RS, int ST, bool PF = false>
 __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_constant__ TileArgs a) {
   using G = TileGeom<TX, TY, TZ>;
-  using M = TileSmem<R, TX, TY, TZ>;
+  constexpr bool kBoth = kBothStates<R, RS>;
+  using M = TileSmem<R, TX, TY, TZ, kBoth>;
   constexpr int SX = G::SX, SY = G::SY;
   constexpr int BX = G::BX, BY = G::BY, NBLK = G::NBLK, NCELL = G::NCELL;
   constexpr int NFX = G::NFX, NFY = G::NFY, NF = G::NF;
@@ -302,7 +339,7 @@ __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_con
   States<R> q(smem_raw + M::Q, G::NS);       // stencil
   States<R> F(smem_raw + M::Q, NF);          // fluxes, once the stencil is traced
   States<R> Ls(smem_raw + M::L, NF);         // lower cell's state at a face
-  States<R> Us(smem_raw + M::U, G::NU);      // upper slab's state at a far face
+  States<R> Us(smem_raw + M::U, M::NUP);     // upper slab's state at a far face (kBoth: upper cell's at a face)
   int32_t* blk = reinterpret_cast<int32_t*>(smem_raw + M::BLK);
   unsigned char* okf = smem_raw + M::OK;
 
@@ -423,18 +460,20 @@ __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_con
   // FP64 code is never contracted and the FP32 forms of hydro_core.cuh spell
   // their contraction out, so any copy of them rounds alike; the other FP32
   // schemes go through one instance of the trace (own cell j = 0, then the
-  // slab cells) and one of the solver per direction, as loops that are not
-  // unrolled (9 % of a Sedov run where it is not needed).
+  // slab cells) and one of the solver (PLMDE: per direction), as loops that are
+  // not unrolled (9 % of a Sedov run where it is not needed).
   constexpr bool kOneSite = sizeof(R) == 4 && !(RS != 0 && (ST == 1 || ST == 2));
   Prim<R> P[3];
-  constexpr int NJ = 1 + (G::NSLAB + NT - 1) / NT;
+  // kBoth: cells and slab cells are one list of items
+  constexpr int NJ = kBoth ? (NCELL + G::NSLAB + NT - 1) / NT : 1 + (G::NSLAB + NT - 1) / NT;
 #pragma unroll (kOneSite ? 1 : 2)
   for (int j = 0; j < NJ; j++) {
     int s = s_own, d = 0, f = 0, r = 0, side = 0;  // slab: slot, direction, face towards the tile
     bool live = code_own != -1;
     unsigned mask = 7u;
-    if (j > 0) {
-      const int it = tid + (j - 1) * NT;
+    const int it = kBoth ? tid + j * NT - NCELL : tid + (j - 1) * NT;
+    const bool cell = kBoth ? it < 0 : j == 0;
+    if (!cell) {
       if (it >= G::NSLAB) break;
       side = it >= G::NU; r = side ? it - G::NU : it;
       if (r < G::NUX) {
@@ -452,23 +491,19 @@ __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_con
       mask = 1u << d;
     }
     if (!live) continue;
-    Prim<R> sp[3], sm[3];
-    trace_slot<R, TX, TY, TZ, RS, ST>(q, s, c, slope_type, dtd, mask, sp, sm);
-    if (j == 0) {
-#pragma unroll
-      for (int k = 0; k < 3; k++) P[k] = sp[k];
-      Ls.put(fx0 + 1, sm[0]);
-      Ls.put(fy0 + TX, sm[1]);
-      Ls.put(fz0 + TX * TY, sm[2]);
-    } else if (side) {  // upper slab: the right state of its face
-      if (d == 0) Us.put(r, sp[0]);
-      else if (d == 1) Us.put(r, sp[1]);
-      else Us.put(r, sp[2]);
-    } else {            // lower slab: the left state
-      if (d == 0) Ls.put(f, sm[0]);
-      else if (d == 1) Ls.put(f, sm[1]);
-      else Ls.put(f, sm[2]);
-    }
+    trace_slot<R, TX, TY, TZ, RS, ST>(q, s, c, slope_type, dtd, mask, [&](int k, const Prim<R>& sp, const Prim<R>& sm) {
+      const int far = k == 0 ? TX : k == 1 ? TX * TY : TX * TY * TZ;  // from a line's first face to its last
+      if (cell) {
+        const int fl = k == 0 ? fx0 : k == 1 ? fy0 : fz0;
+        if (kBoth) Us.put(fl, sp);
+        else P[k] = sp;
+        Ls.put(fl + (k == 0 ? 1 : k == 1 ? TX : TX * TY), sm);
+      } else if (side) {  // upper slab: the right state of its face
+        Us.put(kBoth ? f + far : r, sp);
+      } else {            // lower slab: the left state
+        Ls.put(f, sm);
+      }
+    });
   }
   // difmag > 0 (run-time scheme variant): cmpdivu (uplmde.f90:702-764), the
   // velocity divergence at the cell corners (x-1/2, y-1/2, z-1/2) of the tile,
@@ -531,7 +566,7 @@ __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_con
   // pressure_fix, into Ls[f], which only this thread reads and has read).
   auto face_flux = [&](auto dir, int f, int cx, int cy, int cz, const Prim<R>& L, const Prim<R>& Rr, int fl,
                        Prim<R>& out, R tmp[2]) {
-    constexpr int D = decltype(dir)::value;
+    const int D = dir;
     // refined interface: either neighbour cell refined -> zero flux
     const bool zero_face = (fl & 1) != 0;
     R ql[5], qr[5], fg[6], fo[5];
@@ -626,14 +661,29 @@ __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_con
   };
   // the passes [j0, j1) of every direction
   auto faces = [&](int j0, int j1) {
-    constexpr std::integral_constant<int, 0> DX{};
-    constexpr std::integral_constant<int, 1> DY{};
-    constexpr std::integral_constant<int, 2> DZ{};
+    constexpr Axis<0> DX{};
+    constexpr Axis<1> DY{};
+    constexpr Axis<2> DZ{};
     dir_faces(DX, fx0, j0, min(j1, 1 + (G::NUX + NT - 1) / NT), 0, G::NUX, TY);
     dir_faces(DY, fy0, j0, min(j1, 1 + (G::NUY + NT - 1) / NT), G::NUX, G::NUY, TX);
     dir_faces(DZ, fz0, j0, min(j1, 1 + (G::NUZ + NT - 1) / NT), G::NUX + G::NUY, G::NUZ, TX);
   };
-  if constexpr (kOneSite) {
+  if constexpr (kBoth) {
+    // every face on its own, through one copy of the solvers
+#pragma unroll 1
+    for (int f = tid; f < NF; f += NT) {
+      int d, cx, cy, cz;
+      if (f < NFX) { d = 0; cx = f % (TX + 1); cy = (f / (TX + 1)) % TY; cz = f / ((TX + 1) * TY); }
+      else if (f < NFX + NFY) { const int r = f - NFX; d = 1; cx = r % TX; cy = (r / TX) % (TY + 1); cz = r / (TX * (TY + 1)); }
+      else { const int r = f - NFX - NFY; d = 2; cx = r % TX; cy = (r / TX) % TY; cz = r / (TX * TY); }
+      const int s = (cx + 2) + SX * ((cy + 2) + SY * (cz + 2));
+      const int fl = okf[s] | okf[s - (d == 0 ? 1 : d == 1 ? SX : SX * SY)];
+      if (!(fl & 2)) continue;
+      Prim<R> fo;
+      R t[2];
+      face_flux(d, f, cx, cy, cz, Ls.get(f), Us.get(f), fl, fo, t);
+    }
+  } else if constexpr (kOneSite) {
     faces(0, 1 << 20);
   } else {
     faces(0, 1);        // straight-line code: the three solves overlap
@@ -647,6 +697,14 @@ __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_con
   if (code_own >= 0) {
     const int ch = (x & 1) + 2 * (y & 1) + 4 * (z & 1);
     const int64_t dc = (int64_t)a.ncoarse + (int64_t)code_own * 8 + ch;
+    if (kBoth) {
+      flo[0] = F.get(fx0); flo[1] = F.get(fy0); flo[2] = F.get(fz0);
+      if (PF) {
+        tlo[0][0] = Ls.at(fx0, 0); tlo[0][1] = Ls.at(fx0, 1);
+        tlo[1][0] = Ls.at(fy0, 0); tlo[1][1] = Ls.at(fy0, 1);
+        tlo[2][0] = Ls.at(fz0, 0); tlo[2][1] = Ls.at(fz0, 1);
+      }
+    }
     const Prim<R> fxr = F.get(fx0 + 1), fyr = F.get(fy0 + TX), fzr = F.get(fz0 + TX * TY);
     const R fl[3][5] = {{flo[0].r, flo[0].u, flo[0].v, flo[0].w, flo[0].p},
                         {flo[1].r, flo[1].u, flo[1].v, flo[1].w, flo[1].p},

@@ -291,9 +291,19 @@ bool shape_fits(const rb_context* c, int l, int shape) {
 // FP32-mixed, 852 against 1135, 1155 and 793 us FP64; the 8x8x8 tiles gain in
 // FP64 from some 16 k octs on (27 k octs: 73.8 against 75.8 us, 9 k octs:
 // 36.9 against 34.8). A few hundred octs take one tile's latency, 14-18 us,
-// in any shape.
+// in any shape. The run-time scheme variant has a thread per face, so the
+// latency of its small levels is that of the smallest tile as long as single
+// octs fit in one wave (six of its CTAs per SM; 512 octs, slope type 3: 17 against 22 us
+// FP64, 12.3 against 13.3 us FP32-mixed; acoustic 15 against 19, 12.3 against
+// 14.3), and in FP32-mixed 8x4x4 cells up to some 4 k octs (s3 13.3 against
+// 14.3, acoustic 13.4 against 14.2).
 int default_shape(const rb_context* c, int l, const Level& L) {
-  if (c->precision == RB_PREC_FP64 && L.noct >= 16384 && shape_fits(c, l, 4)) return 4;
+  const bool f64 = c->precision == RB_PREC_FP64;
+  if (rb::scheme_variant(c->hp) == 0) {
+    if (L.noct <= 6 * 148) return 0;
+    if (!f64 && L.noct <= 4096 && shape_fits(c, l, 2)) return 2;
+  }
+  if (f64 && L.noct >= 16384 && shape_fits(c, l, 4)) return 4;
   for (int s : {3, 1})
     if (shape_fits(c, l, s)) return s;
   return 0;

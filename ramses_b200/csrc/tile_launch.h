@@ -28,6 +28,18 @@ constexpr TileShape kTileShapes[kNumTileShapes] = {
     {8, 8, 8, 512},
 };
 
+// The compiled variant of a scheme, 100 * (PLMDE) + 10 * riemann + slope_type;
+// 0: the variant that reads the scheme at run time. The artificial diffusion
+// (difmag > 0) is part of the run-time variant only.
+inline int scheme_variant(const rb_hydro_params& hp) {
+  if (hp.difmag > 0.0 || (hp.slope_type != 1 && hp.slope_type != 2)) return 0;
+  const int r = hp.riemann;
+  if (hp.scheme == RB_SCHEME_MUSCL && (r == RB_RIEMANN_LLF || r == RB_RIEMANN_HLL || r == RB_RIEMANN_HLLC))
+    return 10 * r + hp.slope_type;
+  if (hp.scheme == RB_SCHEME_PLMDE && r == RB_RIEMANN_HLLC) return 100 + 10 * r + hp.slope_type;
+  return 0;
+}
+
 size_t tile_smem_f64(int shape);
 size_t tile_smem_mixed(int shape);
 cudaError_t launch_tile_f64(int shape, const TileArgs& a, int grid, cudaStream_t s);
