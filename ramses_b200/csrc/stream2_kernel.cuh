@@ -246,7 +246,7 @@ __device__ __forceinline__ void stream2_step_body(const StreamArgs& a, const int
     double u[5];
 #pragma unroll
     for (int v = 0; v < 5; v++) u[v] = rp[v * NS + s];
-    return ctoprim_mixed(u, a.hp.smallr, gm1, pfc);
+    return ctoprim_mixed<RS != RB_RIEMANN_HLLC>(u, a.hp.smallr, gm1, pfc);
   };
   auto put_q = [&](int zp, int sq, const Prim<float>& q) {
     const int o = ((zp - zbase) & 1) * NQS + sq;
