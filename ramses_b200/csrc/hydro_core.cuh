@@ -73,12 +73,16 @@ __device__ __forceinline__ Prim<R> ctoprim_cell(const double u[5], const rb_hydr
   if constexpr (sizeof(R) == 4) {
     // FP32-mixed: velocities, E/rho - v^2/2 and its floor in FP64 from a
     // Newton-refined reciprocal; the zero gravity predictor is dropped (it
-    // only changes the sign of a zero velocity)
+    // only changes the sign of a zero velocity). The contraction is spelled
+    // out: a cell in the halo of two tiles is converted by two inlined copies
+    // of this, which have to round alike (see the FP32 forms below)
     const double ir = rcp_newton(q1);
-    const double q2 = u[1] * ir, q3 = u[2] * ir, q4 = u[3] * ir;
-    const double eint = fmx(u[4] * ir - 0.5 * (q2 * q2 + q3 * q3 + q4 * q4), smalle);
+    const double q2 = __dmul_rn(u[1], ir), q3 = __dmul_rn(u[2], ir), q4 = __dmul_rn(u[3], ir);
+    const double v2 = fma(q4, q4, fma(q3, q3, __dmul_rn(q2, q2)));
+    const double eint = fmx(fma(u[4], ir, __dmul_rn(-0.5, v2)), smalle);
     Prim<R> q;
-    q.r = (R)q1; q.u = (R)q2; q.v = (R)q3; q.w = (R)q4; q.p = (R)((gamma - 1.0) * q1 * eint);
+    q.r = (R)q1; q.u = (R)q2; q.v = (R)q3; q.w = (R)q4;
+    q.p = (R)__dmul_rn(__dmul_rn(gamma - 1.0, q1), eint);
     return q;
   }
   // FP64 path: IEEE division as the reference
@@ -694,8 +698,8 @@ __device__ __forceinline__ void from_face(const R f[6], int d, R out[5]) {
 // MUSCL-Hancock predictor, in half slopes. A face at the edge of a tile or
 // column is solved by two CTAs, and often by two inlined copies of this code:
 // the products and sums are written with the contraction spelled out (fmaf,
-// __fmul_rn, __fadd_rn), so that every copy rounds alike and the face has one
-// flux (the FP64 accumulation of the fluxes then telescopes).
+// __fmul_rn, __fadd_rn; also in ctoprim_cell), so that every copy rounds alike
+// and the face has one flux (the FP64 accumulation of the fluxes then telescopes).
 // ---------------------------------------------------------------------------
 // Half slope dq/2 of one variable in one direction (uslope, umuscl.f90:1241-1327):
 // ST = 1 minmod, ST = 2 moncen, in FP32 with the sign applied last.

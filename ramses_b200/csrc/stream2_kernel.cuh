@@ -69,8 +69,11 @@ struct S2Geom {
 // (hydro_core.cuh), with the contraction left to the compiler: one reciprocal
 // per face for the two sound speeds instead of two, and the rounding that
 // long runs of this kernel have been compared at (a strong shock tube
-// amplifies another rounding to 1e-4 in 200 steps). Density products stay
-// above 1e-38 for densities above 1e-19.
+// amplifies another rounding to 1e-4 in 200 steps). That the two copies which
+// solve a face at a column's edge round alike therefore rests on the compiler
+// contracting equal expressions equally, and is held by the tests that these
+// runs conserve to FP64 roundoff. Density products stay above 1e-38 for
+// densities above 1e-19.
 // HLLC flux (riemann_hllc, godunov_utils.f90:988-1209) in FP32 for the mixed
 // path, times dt/dx. Face frame (rho, u_n, P, u_t1, u_t2) in, flux of (mass,
 // normal momentum, energy, t1 momentum, t2 momentum) out. The larger of the
