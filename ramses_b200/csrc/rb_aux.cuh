@@ -510,7 +510,8 @@ static __global__ void __launch_bounds__(RB_RED_NT) reduce_partials_kernel(const
 #define RB_S_TEND (5 * RB_NLV + 5)
 #define RB_S_MAXC (5 * RB_NLV + 6)
 #define RB_S_COARSE (5 * RB_NLV + 7)
-#define RB_S_SIZE (5 * RB_NLV + 8)
+#define RB_S_IDLE (5 * RB_NLV + 8)   // 1 until the run has taken a coarse step: gate of what follows its last one
+#define RB_S_SIZE (5 * RB_NLV + 9)
 
 // Scalar operations, code = op << 8 | level:
 //  GATE     start of a coarse step: raise the done flag if the run is over
@@ -556,7 +557,10 @@ __device__ inline void sched_run(double* __restrict__ s, const SchedProg& p) {
         break;
       case RB_OP_END1: s[RB_S_DTNEW + l - 1] = s[RB_S_DTNEW + l]; break;
       case RB_OP_END2: s[RB_S_DTNEW + l - 1] = s[RB_S_DTOLD + l] + s[RB_S_DTNEW + l]; break;
-      case RB_OP_FINISH: s[RB_S_COARSE] = s[RB_S_COARSE] + 1.0; break;
+      case RB_OP_FINISH:
+        s[RB_S_COARSE] = s[RB_S_COARSE] + 1.0;
+        s[RB_S_IDLE] = 0.0;
+        break;
     }
   }
 }

@@ -1577,6 +1577,7 @@ int level_step_dev(rb_context* c, const LevelStep& st) {
 
 int coarse_step_dev(rb_context* c) {
   const CoarsePlan plan = plan_coarse(c);
+  if (plan.steps.empty()) return sched_impl(c, {(uint16_t)(rb::RB_OP_FINISH << 8), (uint16_t)(rb::RB_OP_GATE << 8)});  // no oct on levelmin
   // with pressure_fix, set_unew (with divu and enew) runs where amr_step has
   // it, at the start of each step of a level with finer octs
   std::vector<char> unew_due(RB_MAXLEVEL + 2, 1);
@@ -1650,6 +1651,8 @@ int sched_upload(rb_context* c, int64_t max_coarse, double t_end) {
   h[RB_S_NSTEP] = (double)c->nstep;
   h[RB_S_TEND] = t_end;
   h[RB_S_MAXC] = (double)max_coarse;
+  h[RB_S_DONE] = !(c->t < t_end) || max_coarse <= 0 ? 1.0 : 0.0;  // a run of no steps changes nothing
+  h[RB_S_IDLE] = 1.0;
   RB_CUDA(cudaMemcpyAsync(c->d_sched, h, RB_S_SIZE * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   return RB_OK;
 }
@@ -1690,7 +1693,11 @@ int run_async_begin(rb_context* c, double t_end, int64_t max_coarse) {
 int run_async_chunk(rb_context* c, int chunk, bool use_graph) { return enqueue_chunk(c, chunk, use_graph); }
 
 int run_async_end(rb_context* c, int64_t* coarse_out) {
-  c->gate = nullptr;
+  struct GateScope {
+    rb_context* c;
+    ~GateScope() { c->gate = nullptr; }
+  } scope{c};
+  c->gate = c->d_sched + RB_S_IDLE;
   // the levels below levelmin are read by no step: one restriction of the
   // final state (adaptive_loop.f90:118-205 restricts after every coarse step)
   for (int l = c->mp.levelmin - 1; l >= 1; l--) RB_TRY(upload_fine_impl(c, l));

@@ -7,7 +7,7 @@ import pytest
 import oracle
 from ramses_b200 import runtime
 
-from helpers import sedov_amr
+from helpers import oct_cells, sedov_amr
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +40,28 @@ def test_subcycling_patterns(cuda_lib, oracle_lib, levels, pattern):
         g = tree.active[lf].astype(np.int64)
         cells = (tree.ncoarse + np.arange(8)[:, None] * tree.ngridmax + g[None, :] - 1).ravel()
         np.testing.assert_array_equal(s.download_unew()[:, cells], orc.uold[:, cells])
+
+
+@pytest.mark.parametrize("pressure_fix", [False, True])
+@pytest.mark.parametrize("stop", ["max_steps", "t_end"])
+def test_run_of_no_steps_changes_nothing(cuda_lib, oracle_lib, stop, pressure_fix):
+    """A run that is over before it starts leaves uold and unew as they are,
+    the levels below levelmin included, which need not be the restriction of
+    the finer ones; the next run's step restricts them."""
+    tree, hp, u = sedov_amr(3, 5)
+    hp.pressure_fix, hp.beta_fix = pressure_fix, 0.5 if pressure_fix else 0.0
+    u = u.copy()
+    low = np.concatenate([(tree.ncoarse + np.arange(8)[:, None] * tree.ngridmax
+                           + tree.active[l].astype(np.int64)[None, :] - 1).ravel() for l in (1, 2)])
+    u[:, low] *= 1.25
+    unew = u * 1.5
+    orc = oracle.OracleRun(tree, hp, u)
+    with runtime.Solver(tree, hp, uold=u) as s:
+        s.upload_unew(unew)
+        assert (s.run(max_steps=0) if stop == "max_steps" else s.run(t_end=s.t, max_steps=5)) == 0
+        np.testing.assert_array_equal(s.download_state(), u)
+        np.testing.assert_array_equal(s.download_unew(), unew)
+        assert s.run(max_steps=1) == 1
+        orc.coarse_step()
+        cells = oct_cells(tree) - 1
+        np.testing.assert_array_equal(s.download_state()[:, cells], orc.uold[:, cells])
