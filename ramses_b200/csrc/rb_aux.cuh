@@ -492,9 +492,10 @@ static __global__ void __launch_bounds__(RB_RED_NT) reduce_partials_kernel(const
 // courant_fine(l) reads at the start of an amr_step(l) is the state that the
 // previous step of level l left (only that step's set_uold and upload_fine
 // write the level's cells), so its wave speeds are taken in the pass that
-// writes it. On a small octree (levels 4-6, 70 launches per coarse step, 2-10
-// us each, mostly launch latency) this and the merged set_unew leave 19:
-// 3.03 -> 2.30 ms per 12 steps; on levels 6-9 (4 M leaf cells), where the
+// writes it. On a small octree (levels 4-6, 52 launches per coarse step, 2-10
+// us each, mostly launch latency) this, the merged set_unew, the one
+// prolongation per two subcycles and the one restriction below levelmin per
+// run leave 23: 3.03 -> 2.30 ms per 12 steps; on levels 6-9 (4 M leaf cells), where the
 // passes saved are memory traffic, 113.0 -> 104.4 ms per 16 steps.
 #define RB_NLV (RB_MAXLEVEL + 2)
 #define RB_S_DTNEW 0
@@ -601,7 +602,7 @@ __device__ __forceinline__ void cfl_tail(double smax, const CflTail& t) {
 
 // The CFL condition of level l's leaf cells in state u: before a run's first
 // step (with unew non-null also set_unew, unew = u), and after each step of a
-// finest level, whose state needs no set_uold pass (see amr_step_dev).
+// finest level, whose state needs no set_uold pass (see level_step_dev).
 // son null: a level without split cells. FAST (FP32-mixed contexts): the wave
 // speed of cfl_speed_fast.
 template <int NT, bool FAST>

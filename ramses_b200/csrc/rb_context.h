@@ -231,7 +231,6 @@ struct rb_context {
   double t = 0.0;
   int64_t nstep = 0;
   int64_t cell_updates = 0;
-  double mass_tot = 0, ekin_tot = 0, eint_tot = 0;
 };
 
 namespace rbi {

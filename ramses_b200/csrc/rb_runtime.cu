@@ -1424,11 +1424,10 @@ int amr_step_impl(rb_context* c, int l, int icount) {
   if (c->lv[l].noct == 0) return RB_OK;
   c->dtold[l] = c->dtnew[l];
   c->dtnew[l] = c->mp.boxlen / c->hp.smallc;
-  double dt_all = c->dtnew[l], ma = 0, ek = 0, ei = 0;
+  double dt_all = c->dtnew[l];
   // a level without finer octs gets set_unew inside its godunov kernel
   const bool fuse = !c->lv[l].has_refined;
-  RB_TRY(courant_impl(c, l, &dt_all, &ma, &ek, &ei, /*with_set_unew=*/!fuse));
-  c->mass_tot += ma; c->ekin_tot += ek; c->eint_tot += ei;
+  RB_TRY(courant_impl(c, l, &dt_all, nullptr, nullptr, nullptr, /*with_set_unew=*/!fuse));
   c->dtnew[l] = rb_min_host(c->dtnew[l], dt_all);
   if (l > c->mp.levelmin)
     c->dtnew[l] = rb_min_host(c->dtnew[l - 1] / (double)(float)c->mp.nsubcycle[l - 1], c->dtnew[l]);
@@ -2109,7 +2108,6 @@ int rb_coarse_step(rb_context* c, double* t_io, double* dtnew_out) {
   oct_changed(c);
   dev_wrote(c);
   if (t_io) c->t = *t_io;
-  c->mass_tot = c->ekin_tot = c->eint_tot = 0.0;
   RB_TRY(amr_step_impl(c, c->mp.levelmin, 1));
   for (int l = c->mp.levelmin - 1; l >= 1; l--) RB_TRY(upload_fine_impl(c, l));
   RB_CUDA(cudaStreamSynchronize(c->stream));
@@ -2447,16 +2445,13 @@ static int uniform_run_tiles(rb_context* c, int nsteps, int use_graph, double* t
   }
   // coarser levels: restriction of the final state (adaptive_loop.f90 + amr_step.f90:442)
   for (int l = lf - 1; l >= 1; l--) RB_TRY(upload_fine_impl(c, l));
-  RB_CUDA(cudaMemcpyAsync(c->h_red, c->d_clock, 6 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  RB_CUDA(cudaMemcpyAsync(c->h_red, c->d_clock, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   RB_CUDA(cudaStreamSynchronize(c->stream));
   if (nsteps > 0) RB_CUDA(cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1));
   c->t = c->h_red[1];
   c->nstep += nsteps;
   c->cell_updates += (int64_t)nsteps * L.leaf_cells;
   c->dtnew[lf] = c->h_red[0];
-  c->mass_tot = c->h_red[2];
-  c->ekin_tot = c->h_red[3];
-  c->eint_tot = c->h_red[4];
   if (t_io) *t_io = c->t;
   if (dt_last_out) *dt_last_out = c->h_red[0];
   return RB_OK;
@@ -2568,16 +2563,13 @@ static int uniform_run_dense(rb_context* c, int nsteps, int use_graph, double* t
     c->dense_cur = (c->dense_cur + nsteps) & 1;
     c->oct_stale = true;
   }
-  RB_CUDA(cudaMemcpyAsync(c->h_red, c->d_clock, 6 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  RB_CUDA(cudaMemcpyAsync(c->h_red, c->d_clock, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   RB_CUDA(cudaStreamSynchronize(c->stream));
   if (nsteps > 0) RB_CUDA(cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1));
   c->t = c->h_red[1];
   c->nstep += nsteps;
   c->cell_updates += (int64_t)nsteps * L.leaf_cells;
   c->dtnew[lf] = c->h_red[0];
-  c->mass_tot = c->h_red[2];
-  c->ekin_tot = c->h_red[3];
-  c->eint_tot = c->h_red[4];
   if (t_io) *t_io = c->t;
   if (dt_last_out) *dt_last_out = c->h_red[0];
   return RB_OK;
