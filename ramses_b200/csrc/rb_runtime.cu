@@ -481,9 +481,10 @@ int build_level_tables(rb_context* c, int l, const std::vector<OctIndex>& idx) {
   // pass 1, tiles in parallel: the source of every block of each tile's
   // stencil box; an absent block that an oct of the tile needs is marked
   // with its father cell f as -1 - f (prolongation entries are numbered in
-  // pass 2)
+  // pass 2). A thread's share is at least 4096 blocks (some 130 us) whatever
+  // the shape.
   std::atomic<int64_t> held{0};  // octs inside the tiles
-  parallel_for(L.ntile, 256, [&](int64_t t0, int64_t t1) {
+  parallel_for(L.ntile, std::max(1, 4096 / NBLK), [&](int64_t t0, int64_t t1) {
     std::vector<char> inner((size_t)TOX * TOY * TOZ);
     int64_t n_inner = 0;
     for (int64_t t = t0; t < t1 && !perr.set.load(); t++) {
@@ -713,12 +714,13 @@ int build_level_tables(rb_context* c, int l, const std::vector<OctIndex>& idx) {
       }
       return k;
     };
-    parallel_for(L.ntile, 1024, [&](int64_t t0, int64_t t1) {
+    const int64_t share = std::max(1, 4096 / NOCT);
+    parallel_for(L.ntile, share, [&](int64_t t0, int64_t t1) {
       for (int64_t t = t0; t < t1; t++) off[t + 1] = tile_entries((int)t, nullptr);
     });
     for (int t = 0; t < L.ntile; t++) off[t + 1] += off[t];
     std::vector<int32_t> ent((size_t)off[L.ntile] * 2);
-    parallel_for(L.ntile, 1024, [&](int64_t t0, int64_t t1) {
+    parallel_for(L.ntile, share, [&](int64_t t0, int64_t t1) {
       for (int64_t t = t0; t < t1; t++) tile_entries((int)t, ent.data() + 2 * (size_t)off[t]);
     });
     RB_TRY(dreserve(c->table_pool, c->stream, &L.d_tile_corr_off, &L.cap_tile_corr_off, off.size()));
