@@ -3,7 +3,7 @@ sm_100a with nvcc (no JIT cache: the .so travels with the source tree).
 
 The FP64 units are compiled with ``--fmad=false`` so that no multiply-add is
 contracted (bit-identical to the reference operation order); the FP32-mixed
-unit uses fast FP32 division/sqrt and contraction.
+units use fast FP32 division/sqrt and contraction.
 """
 from __future__ import annotations
 
@@ -24,7 +24,11 @@ COMMON = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "-
 UNITS = {
     "rb_runtime.cu": ["--fmad=false"],
     "tile_f64.cu": ["--fmad=false"],
+    "tile_f64_pf.cu": ["--fmad=false"],
     "tile_mixed.cu": ["-use_fast_math"],
+    "tile_mixed_pf.cu": ["-use_fast_math"],
+    "stream_f64.cu": ["--fmad=false"],
+    "stream_mixed.cu": ["-use_fast_math"],
     "rb_noalloc.cu": ["--fmad=false"],
     "rb_server.cu": ["--fmad=false"],
 }

@@ -1340,8 +1340,9 @@ rb::TileArgs tile_args(rb_context* c, Level& L, double dt) {
 }
 
 int launch_tile(rb_context* c, int shape, const rb::TileArgs& a, int grid) {
-  cudaError_t e = c->precision == RB_PREC_MIXED ? rb::launch_tile_mixed(shape, a, grid, c->stream)
-                                                : rb::launch_tile_f64(shape, a, grid, c->stream);
+  auto k = c->precision == RB_PREC_MIXED ? (a.divu ? rb::launch_tile_mixed_pf : rb::launch_tile_mixed)
+                                         : (a.divu ? rb::launch_tile_f64_pf : rb::launch_tile_f64);
+  const cudaError_t e = k(shape, a, grid, c->stream);
   if (e != cudaSuccess) return fail(RB_ERR_CUDA, "godunov tile kernel launch failed: %s", cudaGetErrorString(e));
   return RB_OK;
 }

@@ -44,6 +44,9 @@ size_t tile_smem_f64(int shape);
 size_t tile_smem_mixed(int shape);
 cudaError_t launch_tile_f64(int shape, const TileArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_tile_mixed(int shape, const TileArgs& a, int grid, cudaStream_t s);
+// with pressure_fix (a.divu, a.enew and a.corr_tmp set)
+cudaError_t launch_tile_f64_pf(int shape, const TileArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_tile_mixed_pf(int shape, const TileArgs& a, int grid, cudaStream_t s);
 
 // z-streaming kernel of complete levels: column shape (TX x TY cells) and the
 // number of CTAs per SM the register allocation is bounded for. Shapes 5 and
