@@ -296,12 +296,15 @@ bool shape_fits(const rb_context* c, int l, int shape) {
 // octs fit in one wave (six of its CTAs per SM; 512 octs, slope type 3: 17 against 22 us
 // FP64, 12.3 against 13.3 us FP32-mixed; acoustic 15 against 19, 12.3 against
 // 14.3), and in FP32-mixed 8x4x4 cells up to some 4 k octs (s3 13.3 against
-// 14.3, acoustic 13.4 against 14.2).
+// 14.3, acoustic 13.4 against 14.2). Its FP64 8x8x4 tiles run one per SM, so
+// 8x8x8 cells take over where those need a second wave (7 k octs: acoustic 36
+// against 42 us, exact 54 against 60; 4 k octs: 23.5 against 19.4, 42 against 34).
 int default_shape(const rb_context* c, int l, const Level& L) {
   const bool f64 = c->precision == RB_PREC_FP64;
   if (rb::scheme_variant(c->hp) == 0) {
     if (L.noct <= 6 * 148) return 0;
     if (!f64 && L.noct <= 4096 && shape_fits(c, l, 2)) return 2;
+    if (f64 && L.noct > 32 * 148 && shape_fits(c, l, 4)) return 4;
   }
   if (f64 && L.noct >= 16384 && shape_fits(c, l, 4)) return 4;
   for (int s : {3, 1})
