@@ -216,12 +216,19 @@ constexpr size_t tile_smem_bytes() {
   return TileSmem<R, TX, TY, TZ, BOTH>::SIZE;
 }
 
+// The FP32 forms for minmod and moncen and the run-time variant hand each
+// direction's face states to their place as they are formed; the others store
+// them after the trace (FP64 hllc with minmod spills 64 bytes so, 88 the other
+// way; FP32-mixed, 8 bytes and none).
+template <typename R, int RS, int ST>
+constexpr bool kPutEach = kBothStates<R, RS> || (sizeof(R) == 4 && RS != 0 && (ST == 1 || ST == 2));
+
 // Traced face states of one cell from its state q0 and its neighbours in q
 // (stencil slot s): sp[d] at the lower, sm[d] at the upper face of direction d,
-// for the directions of mask, each handed to put(d, sp, sm).
+// for the directions of mask; with kPutEach, handed to put(d, sp, sm).
 template <typename R, int TX, int TY, int TZ, int RS, int ST, typename Put>
 __device__ __forceinline__ void trace_slot(const States<R>& q, int s, const Consts<R>& c, int slope_type,
-                                           const R dtd[3], unsigned mask, Put&& put) {
+                                           const R dtd[3], unsigned mask, Prim<R> sp[3], Prim<R> sm[3], Put&& put) {
   using G = TileGeom<TX, TY, TZ>;
   constexpr int st[3] = {1, G::SX, G::SX * G::SY};
   const Prim<R> q0 = q.get(s);
@@ -295,7 +302,6 @@ __device__ __forceinline__ void trace_slot(const States<R>& q, int s, const Cons
         dq[v][0] = slop * dq[v][0]; dq[v][1] = slop * dq[v][1]; dq[v][2] = slop * dq[v][2];
       }
     }
-    Prim<R> sp[3], sm[3];
     if constexpr (kBothStates<R, RS>) {
       // a direction at a time: the two predictors meet with one pair of states live, not three
 #pragma unroll
@@ -306,9 +312,6 @@ __device__ __forceinline__ void trace_slot(const States<R>& q, int s, const Cons
       }
     } else {
       trace_sel<R, RS, ST>(q0, dq, c, dtd, sp, sm, mask);
-#pragma unroll
-      for (int d = 0; d < 3; d++)
-        if (mask & (1u << d)) put(d, sp[d], sm[d]);
     }
   }
 }
@@ -471,9 +474,9 @@ __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_con
     int s = s_own, d = 0, f = 0, r = 0, side = 0;  // slab: slot, direction, face towards the tile
     bool live = code_own != -1;
     unsigned mask = 7u;
-    const int it = kBoth ? tid + j * NT - NCELL : tid + (j - 1) * NT;
-    const bool cell = kBoth ? it < 0 : j == 0;
+    const bool cell = kBoth ? tid + j * NT < NCELL : j == 0;
     if (!cell) {
+      const int it = kBoth ? tid + j * NT - NCELL : tid + (j - 1) * NT;
       if (it >= G::NSLAB) break;
       side = it >= G::NU; r = side ? it - G::NU : it;
       if (r < G::NUX) {
@@ -491,7 +494,7 @@ __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_con
       mask = 1u << d;
     }
     if (!live) continue;
-    trace_slot<R, TX, TY, TZ, RS, ST>(q, s, c, slope_type, dtd, mask, [&](int k, const Prim<R>& sp, const Prim<R>& sm) {
+    auto put = [&](int k, const Prim<R>& sp, const Prim<R>& sm) {
       const int far = k == 0 ? TX : k == 1 ? TX * TY : TX * TY * TZ;  // from a line's first face to its last
       if (cell) {
         const int fl = k == 0 ? fx0 : k == 1 ? fy0 : fz0;
@@ -503,7 +506,26 @@ __global__ void __launch_bounds__(NT, MINB) godunov_tile_kernel(const __grid_con
       } else {            // lower slab: the left state
         Ls.put(f, sm);
       }
-    });
+    };
+    Prim<R> sp[3], sm[3];
+    trace_slot<R, TX, TY, TZ, RS, ST>(q, s, c, slope_type, dtd, mask, sp, sm, put);
+    if constexpr (!kPutEach<R, RS, ST>) {
+      if (cell) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) P[k] = sp[k];
+        Ls.put(fx0 + 1, sm[0]);
+        Ls.put(fy0 + TX, sm[1]);
+        Ls.put(fz0 + TX * TY, sm[2]);
+      } else if (side) {
+        if (d == 0) Us.put(r, sp[0]);
+        else if (d == 1) Us.put(r, sp[1]);
+        else Us.put(r, sp[2]);
+      } else {
+        if (d == 0) Ls.put(f, sm[0]);
+        else if (d == 1) Ls.put(f, sm[1]);
+        else Ls.put(f, sm[2]);
+      }
+    }
   }
   // difmag > 0 (run-time scheme variant): cmpdivu (uplmde.f90:702-764), the
   // velocity divergence at the cell corners (x-1/2, y-1/2, z-1/2) of the tile,
